@@ -260,7 +260,7 @@ def render_scene(which):
 
 
 # Algorithmic bytes of the wavefront path tracer, per event (the fixed record sizes its kernels
-# read and write; traversal bytes come from counted nodes and leaf records, 80 B and 48 B):
+# read and write; traversal bytes come from counted nodes and leaf records, 96 B and 48 B):
 #   camera path (k_raygen: ray 32 + throughput 16 + radiance 16 + queue 4; k_film: radiance 16)
 #   extension ray (k_extend: queue 4 + ray 32 + hit 8 + class queue 4)
 #   shaded vertex (k_shade: class queue 4 + hit 8 + ray 32 + throughput 16 + leaf record 48 +
@@ -269,7 +269,7 @@ def render_scene(which):
 #   shadow ray (k_shade writes and k_shadow reads its 48 B record)
 #   pixel (k_film: 12 B of RGB film written)
 PT_BYTES = {"path": 68 + 16, "extension_ray": 48, "shaded_vertex": 156, "continuation": 52, "shadow_ray": 96,
-            "pixel": 12, "node": 80, "leaf_record": 48}
+            "pixel": 12, "node": 96, "leaf_record": 48}
 
 
 def path_tracer_bytes(st, pixels):
@@ -823,7 +823,7 @@ def main():
     l2_peak = ctx.l2_read_bandwidth(32 << 20, 50)
     # algorithmic traffic of one launch
     nodes, recs = ctx.trace_counts_dev(d_rays.data_ptr(), n)
-    alg_bytes = n * (32 + 8) + nodes * 80 + recs * 48
+    alg_bytes = n * (32 + 8) + nodes * 96 + recs * 48
     avg_launch_s = statistics.mean(launch_ms) / 1e3
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / avg_launch_s / 1e9

@@ -121,7 +121,7 @@ typedef struct rbr_scene_stats {
     uint32_t num_primitives;      /* all primitives */
     uint32_t num_bounded;         /* primitives inside the BVH */
     uint32_t num_unbounded;       /* planes, tested outside the BVH */
-    uint32_t num_wide_nodes;      /* 8-wide nodes (80 B each) */
+    uint32_t num_wide_nodes;      /* 8-wide nodes (96 B each) */
     uint32_t num_leaf_records;    /* leaf primitive records (48 B each) */
     uint32_t max_depth;           /* depth of the wide tree */
     uint32_t wrapped_leaves;      /* leaves given a wide node of their own: a node beside internal
@@ -262,8 +262,8 @@ rbr_status rbr_scene_stats_get(const rbr_ctx* ctx, rbr_scene_stats* out);
  *                          between two sets of path buffers on two streams; an image that
  *                          fits one wave is rendered as two half-image waves; when the second
  *                          set cannot be allocated, the waves run one at a time in the first)
- *   "trace.node_test"      sorted queries of kernel 0: 0 the packed node test (f32x2 FMAs), 1 a
- *                          register-lean one (scalar FMAs, fewer live registers)
+ *   "trace.node_test"      0 or 1; kept for programs that set it: every kernel runs the one node
+ *                          test there is
  *   "trace.stream_io"      kernel 0: rays read and hits written with evict-first hints (default 1)
  *   "trace.l2_persist"     kernel 0: 1 reserves the largest persisting-L2 set-aside this process's
  *                          context allows and marks the BVH (nodes and leaf records) persisting for
@@ -295,7 +295,7 @@ rbr_status rbr_scene_stats_get(const rbr_ctx* ctx, rbr_scene_stats* out);
 rbr_status rbr_param_set(rbr_ctx* ctx, const char* name, int64_t value);
 rbr_status rbr_param_get(const rbr_ctx* ctx, const char* name, int64_t* value);
 /* Autotuner (no reference counterpart): times the traversal variants ("trace.kernel",
- * "trace.min_blocks", "trace.order" 0, 4 and 5, "trace.node_test") on n rays of the caller's own
+ * "trace.min_blocks", "trace.order" 0, 4 and 5) on n rays of the caller's own
  * workload (device pointer) against the uploaded scene, keeps the fastest in the context and
  * returns its time per launch in microseconds (out_us may be NULL). Waits for the timings. */
 rbr_status rbr_autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, int64_t* out_us);
@@ -316,7 +316,7 @@ rbr_status rbr_trace_host(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
 /* Diagnostic: replays the traversal of n rays (device pointer) and returns the total number of
  * 8-wide nodes fetched (out[0]) and leaf records tested (out[1]); waits for the result.
  * The traversal order of a ray is deterministic, so these are its algorithmic node and leaf
- * traffic (80 B per node, 48 B per record) for roofline accounting. No reference counterpart. */
+ * traffic (96 B per node, 48 B per record) for roofline accounting. No reference counterpart. */
 rbr_status rbr_trace_counts(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, uint64_t out[2]);
 
 /* Renders the scene with the wavefront path tracer.

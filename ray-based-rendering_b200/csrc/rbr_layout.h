@@ -1,6 +1,17 @@
-// Device memory layout of a scene (shared by the host builder and the kernels).
+// Memory layout of a scene (shared by the host builder and the kernels).
 //
-// Wide BVH node (80 B, five 16 B words, 16 B aligned):
+// Wide BVH node in device memory (96 B, three 32 B sectors, each read by one 256-bit load):
+//   w0-w2    px, py, pz (f32): biased origin of the node's quantisation grid (as below)
+//   w3       imask (bits 0-7): slots that hold an internal node
+//   w4, w5   child_base, prim_base
+//   w6, w7   per slot byte of a leaf: (records << 5) | offset of its first record from prim_base
+//   w8-w19   per axis qlo[8], qhi[8]: child boxes in 8-bit grid coordinates
+//   w20, w21 byte o: imask in the visiting order of octant o (bit j set if slot j ^ o is internal)
+//   w22      grid steps of x (low half) and y (high half) as BF16 (powers of two, so exact)
+//   w23      grid step of z as f32
+// device_node() makes it from the builder's node:
+//
+// Wide BVH node of the builder (80 B, five 16 B words):
 //   word0  px, py, pz (f32)      biased origin of the node's quantisation grid: plane byte q of
 //                                axis k lies at p_k + (kGridBias + q) * 2^(e_k - 127), so one
 //                                byte permute of q into the mantissa of 32768.0f gives the
@@ -44,7 +55,8 @@ constexpr uint32_t kPrimPlane = 3;
 constexpr uint32_t kTypeShift = 30;
 constexpr uint32_t kIdMask = (1u << kTypeShift) - 1;
 
-constexpr int kNodeWords = 20;   // u32 words per wide node
+constexpr int kNodeWords = 20;     // u32 words per wide node of the builder
+constexpr int kDevNodeWords = 24;  // u32 words per wide node in device memory
 constexpr int kRecordWords = 12; // u32 words per leaf record
 constexpr int kMaxLeafPrims = 4;
 constexpr int kStackSize = 64;   // traversal stack entries; the builder keeps the tree shallower
@@ -61,5 +73,28 @@ constexpr float kEpsilon = 1e-4f;
 constexpr int kErrStackOverflow = 1;
 constexpr int kErrQueueOverflow = 2;
 constexpr int kErrDeviceTimeout = 4;  // a bounded wait (tensor-core completion) ran out
+
+// The device form of a builder node.
+inline void device_node(const uint32_t* w, uint32_t* out) {
+    const uint32_t imask = w[3] >> 24;
+    uint32_t step[3], perm[8];
+    for (int a = 0; a < 3; ++a) step[a] = ((w[3] >> (8 * a)) & 0xFFu) << 23;  // 2^(e - 127) as f32 bits
+    for (uint32_t o = 0; o < 8; ++o) {
+        perm[o] = 0;
+        for (uint32_t j = 0; j < 8; ++j) perm[o] |= ((imask >> (j ^ o)) & 1u) << j;
+    }
+    for (int a = 0; a < 3; ++a) out[a] = w[a];
+    out[3] = imask;
+    for (int k = 4; k < 8; ++k) out[k] = w[k];
+    for (int a = 0; a < 3; ++a)
+        for (int k = 0; k < 2; ++k) {
+            out[8 + 4 * a + k] = w[8 + 2 * a + k];
+            out[10 + 4 * a + k] = w[14 + 2 * a + k];
+        }
+    out[20] = perm[0] | perm[1] << 8 | perm[2] << 16 | perm[3] << 24;
+    out[21] = perm[4] | perm[5] << 8 | perm[6] << 16 | perm[7] << 24;
+    out[22] = (step[0] >> 16) | (step[1] & 0xFFFF0000u);
+    out[23] = step[2];
+}
 
 }  // namespace rbr

@@ -41,12 +41,14 @@ struct LightDev {
 
 // Everything a kernel needs to read a scene. Passed by value.
 struct DeviceScene {
-    const uint4* nodes;      // kNodeWords/4 uint4 per node
+    const uint4* nodes;      // kDevNodeWords/4 uint4 per node
     const float4* records;   // 3 float4 per leaf record
     const float4* planes;    // per plane: (unit normal, d)
     const uint32_t* plane_tags;
     uint32_t num_nodes;
     uint32_t num_planes;
+    float tree_centre[3];    // centre of the BVH's box, and the sum of its half extents
+    float tree_reach;
     // shading data, indexed by primitive id
     const uint32_t* prim_record;   // leaf record index, or (plane index | 0x80000000)
     const uint32_t* prim_material;

@@ -388,18 +388,31 @@ rbr_status upload_scene(rbr_ctx* ctx, const rbr_scene_desc* d) {
     DeviceScene s{};
     void* p = nullptr;
     rbr_status st;
-    // nodes and leaf records in one allocation (records right after the nodes, 16-byte aligned
-    // since a node is 80 bytes): the traversal's whole read set is one address range, which an
+    // nodes and leaf records in one allocation (records right after the nodes, 32-byte aligned
+    // since a device node is 96 bytes): the traversal's whole read set is one address range, which an
     // L2 access-policy window can cover ("trace.l2_persist")
     {
-        std::vector<uint32_t> bvh_words(bvh.nodes.size() + records.size());
-        std::copy(bvh.nodes.begin(), bvh.nodes.end(), bvh_words.begin());
-        std::copy(records.begin(), records.end(), bvh_words.begin() + static_cast<std::ptrdiff_t>(bvh.nodes.size()));
+        const size_t nn = bvh.nodes.size() / kNodeWords, node_words = nn * kDevNodeWords;
+        std::vector<uint32_t> bvh_words(node_words + records.size());
+        for (size_t i = 0; i < nn; ++i) device_node(&bvh.nodes[i * kNodeWords], &bvh_words[i * kDevNodeWords]);
+        std::copy(records.begin(), records.end(), bvh_words.begin() + static_cast<std::ptrdiff_t>(node_words));
         if ((st = upload(ctx, bvh_words, "BVH nodes and leaf records", &p)) != RBR_OK) return free_scene(ctx), st;
         s.nodes = bvh.nodes.empty() ? nullptr : static_cast<const uint4*>(p);
-        s.records = records.empty() ? nullptr : reinterpret_cast<const float4*>(static_cast<const uint32_t*>(p) + bvh.nodes.size());
+        s.records = records.empty() ? nullptr : reinterpret_cast<const float4*>(static_cast<const uint32_t*>(p) + node_words);
         ctx->bvh_base = p;
         ctx->bvh_bytes = bvh_words.size() * 4;
+        if (nn) {  // the tree's box from the root's quantisation grid (every child plane lies on it)
+            const uint32_t* w = bvh.nodes.data();
+            double reach = 0.0;
+            for (int a = 0; a < 3; ++a) {
+                float org;
+                std::memcpy(&org, &w[a], 4);
+                const double step = std::ldexp(1.0, static_cast<int>((w[3] >> (8 * a)) & 0xFFu) - 127);
+                s.tree_centre[a] = static_cast<float>(org + (kGridBias + 127.5) * step);
+                reach += 128.0 * step;
+            }
+            s.tree_reach = static_cast<float>(reach * 1.001);
+        }
     }
     if ((st = upload(ctx, planes, "planes", &p)) != RBR_OK) return free_scene(ctx), st;
     s.planes = static_cast<const float4*>(p);

@@ -45,7 +45,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks) k_trace_closest(Devic
 // The same query on the rays in the order `perm` (a permutation of 0..n-1): rays that start
 // close together with directions of the same octant share warps, so they walk the same nodes.
 // Answers go to the rays' own positions.
-template <int kMinBlocks, bool kStream, bool kLean = false>
+template <int kMinBlocks, bool kStream>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_trace_closest_perm(DeviceScene s, const float4* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ perm,
                          uint2* __restrict__ hits, int* err) {
@@ -55,7 +55,7 @@ __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     const float4 a = ray_word<kStream>(rays + 2 * static_cast<size_t>(i));
     const float4 b = ray_word<kStream>(rays + 2 * static_cast<size_t>(i) + 1);
     float t = 0.0f;
-    const uint32_t prim = traverse<false, false, kLean>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, t, err);
+    const uint32_t prim = traverse<false>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, t, err);
     put_hit<kStream>(hits + i, make_uint2(prim, prim == 0xFFFFFFFFu ? 0u : __float_as_uint(t)));
 }
 
@@ -217,6 +217,14 @@ __device__ __forceinline__ uint32_t lane_mask_lt() {
     return m;
 }
 
+// The answer of a finished TraceState for ray idx.
+template <bool kAny>
+__device__ __forceinline__ void put_answer(uint2* hits, uint8_t* occ, uint32_t idx, const TraceState& st, uint32_t anyhit) {
+    if (kAny) occ[idx] = static_cast<uint8_t>(anyhit);
+    else hits[idx] = make_uint2(st.best < 0 ? 0xFFFFFFFFu : static_cast<uint32_t>(st.best),
+                                st.best < 0 ? 0u : __float_as_uint(st.tbest));
+}
+
 // Persistent warps: each warp takes chunks of kChunk consecutive rays from a global cursor
 // (one atomic per chunk) and hands the next ray of its chunk to any lane whose ray is done,
 // so lanes keep working while the warp's other rays are still traversing. Every loop
@@ -260,9 +268,7 @@ __global__ void __launch_bounds__(kPersistBlock) k_trace_persist(DeviceScene s, 
                 const float4 a = __ldg(rays + 2 * static_cast<size_t>(idx));
                 const float4 b = __ldg(rays + 2 * static_cast<size_t>(idx) + 1);
                 if (trace_begin<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, st, anyhit)) {
-                    if (kAny) occ[idx] = static_cast<uint8_t>(anyhit);
-                    else hits[idx] = make_uint2(st.best < 0 ? 0xFFFFFFFFu : static_cast<uint32_t>(st.best),
-                                                st.best < 0 ? 0u : __float_as_uint(st.tbest));
+                    put_answer<kAny>(hits, occ, idx, st, anyhit);
                     idx = 0xFFFFFFFFu;  // finished at once: takes another ray in this round
                 }
             }
@@ -272,52 +278,33 @@ __global__ void __launch_bounds__(kPersistBlock) k_trace_persist(DeviceScene s, 
         const bool active = idx != 0xFFFFFFFFu;
         if (__ballot_sync(0xFFFFFFFFu, active) == 0) break;  // only when the rays are exhausted
         if (active && trace_step<kAny>(s, st, stack, err, anyhit)) {
-            if (kAny) occ[idx] = static_cast<uint8_t>(anyhit);
-            else hits[idx] = make_uint2(st.best < 0 ? 0xFFFFFFFFu : static_cast<uint32_t>(st.best),
-                                        st.best < 0 ? 0u : __float_as_uint(st.tbest));
+            put_answer<kAny>(hits, occ, idx, st, anyhit);
             idx = 0xFFFFFFFFu;
         }
     }
 }
 
 // ------------------------------------------------------------------------------------------
-// Warp-cooperative traversal: a group of 8 lanes traces one ray (4 rays per warp). In a node
-// step lane j tests child slot j of the node and the group ORs the slots' bits of the node's
-// hit mask (internal children and leaf records) with shuffles; in a leaf step the lanes test up to 8
-// of the node's leaf records at once and keep the closest with a shuffle min-reduction
-// (key = t bits, then the highest id). Group state is replicated in the 8 lanes, so the group
-// never diverges internally; the short stack lives in shared memory (all 8 lanes write the
-// same entry and read back their own write, so no cross-lane synchronisation is needed).
+// Warp-cooperative traversal: a group of 8 lanes traces one ray (4 rays per warp; group_step in
+// rbr_device.cuh) and takes the next ray of the warp's chunk when its own is done.
 // ------------------------------------------------------------------------------------------
 constexpr int kCoopBlock = 128;
-constexpr int kCoopGroups = kCoopBlock / 8;
-
-__device__ __forceinline__ uint32_t nth_set_bit(uint32_t m, int n) {  // n-th (0-based) set bit, or 32
-    for (int k = 0; k < n && m; ++k) m &= m - 1;
-    return m ? static_cast<uint32_t>(__ffs(m) - 1) : 32u;
-}
 
 template <bool kAny>
 __global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const float4* __restrict__ rays, uint32_t n,
                                                            uint2* __restrict__ hits, uint8_t* __restrict__ occ,
                                                            int* err, uint32_t* cursor) {
-    __shared__ uint2 sstack[kCoopGroups][kStackSize];
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t j = lane & 7u;             // slot / record lane within the group
-    const uint32_t g = lane >> 3;             // group within the warp
-    const uint32_t gmask = 0xFFu << (8 * g);  // the group's lanes
-    uint2* stack = sstack[threadIdx.x >> 3];
+    const GroupLanes g = group_lanes();
     uint32_t chunk_next = 0, chunk_end = 0;   // warp-uniform
     bool exhausted = false;                   // warp-uniform
     uint32_t idx = 0xFFFFFFFFu;               // group-uniform
-    RayCtx r;
-    float tbest = 0.0f;
-    int best = -1;
-    uint2 ng = make_uint2(0, 0), pg = make_uint2(0, 0);
-    int sp = 0;
+    uint32_t anyhit = 0;
+    TraceState st{};
+    uint2 stack[kStackSize];
     while (true) {
         // give idle groups new rays from the warp's chunk
-        uint32_t need = __ballot_sync(0xFFFFFFFFu, j == 0 && idx == 0xFFFFFFFFu);
+        uint32_t need = __ballot_sync(0xFFFFFFFFu, g.j == 0 && idx == 0xFFFFFFFFu);
         while (need != 0 && !exhausted) {
             if (chunk_next == chunk_end) {
                 uint32_t b = 0;
@@ -331,117 +318,22 @@ __global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const 
                 chunk_end = min(b + kChunk, n);
             }
             const uint32_t avail = chunk_end - chunk_next;
-            const uint32_t rank = __popc(need & ((1u << (8 * g)) - 1u));
-            if (((need >> (8 * g)) & 1u) && rank < avail) {
+            const uint32_t rank = __popc(need & ((1u << g.shift) - 1u));
+            if (((need >> g.shift) & 1u) && rank < avail) {
                 idx = chunk_next + rank;
                 const float4 a = __ldg(rays + 2 * static_cast<size_t>(idx));
                 const float4 b = __ldg(rays + 2 * static_cast<size_t>(idx) + 1);
-                const f3 o = mk(a.x, a.y, a.z), d = mk(b.x, b.y, b.z);
-                tbest = a.w;
-                best = -1;
-                bool done = false;
-                for (uint32_t i = 0; i < s.num_planes && !done; ++i) {
-                    const float4 pl = __ldg(s.planes + i);
-                    const float t = hit_plane(o, d, mk(pl.x, pl.y, pl.z), pl.w, tbest);
-                    if (t >= 0.0f) {
-                        const uint32_t id = __ldg(s.plane_tags + i) & kIdMask;
-                        if (kAny) done = true;
-                        else if (accept(t, id, tbest, best)) {
-                            tbest = t;
-                            best = static_cast<int>(id);
-                        }
-                    }
-                }
-                if (kAny && done) {
-                    if (j == 0) occ[idx] = 1;
-                    idx = 0xFFFFFFFFu;
-                } else if (s.num_nodes == 0) {
-                    if (j == 0) {
-                        if (kAny) occ[idx] = 0;
-                        else hits[idx] = make_uint2(best < 0 ? 0xFFFFFFFFu : static_cast<uint32_t>(best),
-                                                    best < 0 ? 0u : __float_as_uint(tbest));
-                    }
-                    idx = 0xFFFFFFFFu;
-                } else {
-                    r = make_ctx(o, d);
-                    sp = 0;
-                    pg = make_uint2(0, 0);
-                    // a pseudo node group whose only child is the root (slot 0, internal)
-                    ng = make_uint2(0u, (1u << (24 + (0u ^ r.oct))) | (1u << 16));
+                if (trace_begin<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, st, anyhit)) {
+                    if (g.j == 0) put_answer<kAny>(hits, occ, idx, st, anyhit);
+                    idx = 0xFFFFFFFFu;  // finished at once: takes another ray in this round
                 }
             }
             chunk_next += min(__popc(need), avail);
-            need = __ballot_sync(0xFFFFFFFFu, j == 0 && idx == 0xFFFFFFFFu);
+            need = __ballot_sync(0xFFFFFFFFu, g.j == 0 && idx == 0xFFFFFFFFu);
         }
         if (__ballot_sync(0xFFFFFFFFu, idx != 0xFFFFFFFFu) == 0) break;  // rays exhausted
-        if (idx == 0xFFFFFFFFu) continue;
-        bool finished = false;
-        uint32_t anyres = 0;
-        if (pg.y != 0) {
-            // leaf step: up to 8 records at once
-            const uint32_t bit = nth_set_bit(pg.y, static_cast<int>(j));
-            unsigned long long key = ~0ull;
-            if (bit < 32) {
-                uint32_t tag;
-                const float t = hit_record(s.records, pg.x + bit, r.o, r.d, tbest, tag);
-                if (t >= 0.0f) key = (static_cast<unsigned long long>(__float_as_uint(t)) << 32) | (~(tag & kIdMask));
-            }
-            if (kAny) {
-                if (__ballot_sync(gmask, key != ~0ull) != 0) {
-                    finished = true;
-                    anyres = 1;
-                }
-            } else {
-                for (int off = 1; off < 8; off <<= 1) {
-                    const unsigned long long o2 = __shfl_xor_sync(gmask, key, off, 8);
-                    key = o2 < key ? o2 : key;
-                }
-                if (key != ~0ull) {
-                    const float t = __uint_as_float(static_cast<uint32_t>(key >> 32));
-                    const uint32_t id = ~static_cast<uint32_t>(key) & kIdMask;
-                    if (accept(t, id, tbest, best)) {
-                        tbest = t;
-                        best = static_cast<int>(id);
-                    }
-                }
-            }
-            // drop the (up to) 8 records just tested
-            pg.y = __popc(pg.y) <= 8 ? 0u : pg.y & ~((2u << nth_set_bit(pg.y, 7)) - 1u);
-        } else {
-            // node step (after a pop if the current group is exhausted)
-            if ((ng.y & 0xFF000000u) == 0) {
-                if (sp == 0) {
-                    finished = true;
-                } else {
-                    ng = stack[--sp];
-                }
-            }
-            if (!finished) {
-                const int b = 31 - __clz(ng.y);
-                ng.y &= ~(1u << b);
-                const uint32_t slot = static_cast<uint32_t>(b - 24) ^ r.oct;
-                const uint32_t imask_p = (ng.y >> 16) & 0xFFu;
-                const uint32_t child = ng.x + __popc(imask_p & ((1u << slot) - 1u));
-                if (ng.y & 0xFF000000u) {
-                    if (sp < kStackSize) stack[sp++] = ng;
-                    else atomicOr(err, kErrStackOverflow);
-                }
-                // lane j tests slot j; the group ORs the slots' bits of the node's hit mask
-                const NodeView v = node_view(s.nodes, child, r);
-                const int jj = static_cast<int>(j);
-                uint32_t bits = slot_hit(v, jj, tbest) ? slot_bits(v, jj) : 0u;
-                bits |= __shfl_xor_sync(gmask, bits, 1, 8);
-                bits |= __shfl_xor_sync(gmask, bits, 2, 8);
-                bits |= __shfl_xor_sync(gmask, bits, 4, 8);
-                split_hits(v, bits, ng, pg);
-            }
-        }
-        if (finished) {
-            if (j == 0) {
-                if (kAny) occ[idx] = static_cast<uint8_t>(anyres);
-                else hits[idx] = make_uint2(best < 0 ? 0xFFFFFFFFu : static_cast<uint32_t>(best),
-                                            best < 0 ? 0u : __float_as_uint(tbest));
-            }
+        if (idx != 0xFFFFFFFFu && group_step<kAny>(s, g, st, stack, err, anyhit)) {
+            if (g.j == 0) put_answer<kAny>(hits, occ, idx, st, anyhit);
             idx = 0xFFFFFFFFu;
         }
     }
@@ -559,10 +451,7 @@ cudaError_t launch_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_
             auto* h = static_cast<uint2*>(out);
             const bool st = ctx->trace_stream_io != 0;
             const int mb = ctx->trace_min_blocks;
-            auto k = ctx->trace_node_test == 1
-                         ? (mb >= 12 ? k_trace_closest_perm<12, true, true>
-                            : mb >= 10 ? k_trace_closest_perm<10, true, true> : k_trace_closest_perm<8, true, true>)
-                     : mb >= 12 ? (st ? k_trace_closest_perm<12, true> : k_trace_closest_perm<12, false>)
+            auto k = mb >= 12 ? (st ? k_trace_closest_perm<12, true> : k_trace_closest_perm<12, false>)
                      : mb >= 10 ? (st ? k_trace_closest_perm<10, true> : k_trace_closest_perm<10, false>)
                                 : (st ? k_trace_closest_perm<8, true> : k_trace_closest_perm<8, false>);
             return launch_query(ctx, k, blocks, stream, ctx->scene, r, n, perm, h, ctx->d_error);
@@ -605,18 +494,16 @@ cudaError_t launch_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_
 // Times every traversal variant on the caller's rays (device pointer) and keeps the fastest.
 rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, int64_t* chosen_ms_x1000) {
     struct Cand {
-        int kernel, min_blocks, per_sm, order, node_test;
+        int kernel, min_blocks, per_sm, order;
     };
     // Unsorted variants, and sorted ones with the 16-bit keys of orders 4 and 5 (the counting
-    // sort of this file) and either node test. Orders 1-3 (CUB's radix sort) stay selectable
-    // by parameter; measured slower than orders 4 and 5, they are not candidates.
-    const Cand cands[] = {{0, 8, 0, 0, 0},  {0, 10, 0, 0, 0}, {0, 12, 0, 0, 0}, {1, 10, 0, 0, 0}, {2, 10, 0, 0, 0},
-                          {0, 8, 0, 4, 0},  {0, 10, 0, 4, 0}, {0, 10, 0, 5, 0}, {0, 12, 0, 5, 0}, {0, 8, 0, 5, 1},
-                          {0, 10, 0, 4, 1}, {0, 10, 0, 5, 1}, {0, 12, 0, 5, 1}, {1, 10, 0, 5, 0}};
+    // sort of this file). Orders 1-3 (CUB's radix sort) stay selectable by parameter; measured
+    // slower than orders 4 and 5, they are not candidates.
+    const Cand cands[] = {{0, 8, 0, 0}, {0, 10, 0, 0}, {0, 12, 0, 0}, {1, 10, 0, 0}, {2, 10, 0, 0}, {0, 8, 0, 4},
+                          {0, 10, 0, 4}, {0, 12, 0, 4}, {0, 8, 0, 5}, {0, 10, 0, 5}, {0, 12, 0, 5}, {1, 10, 0, 5}};
     rbr_status st = ensure(ctx, ctx->stage_out, size_t(n) * (any_hit ? 1 : sizeof(rbr_hit)), "autotune output");
     if (st != RBR_OK) return st;
-    const Cand saved{ctx->trace_kernel, ctx->trace_min_blocks, ctx->trace_blocks_per_sm, ctx->trace_order,
-                     ctx->trace_node_test};
+    const Cand saved{ctx->trace_kernel, ctx->trace_min_blocks, ctx->trace_blocks_per_sm, ctx->trace_order};
     float best_ms = 1e30f;
     Cand best = saved;
     cudaEvent_t a, b;
@@ -627,7 +514,6 @@ rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
         ctx->trace_min_blocks = c.min_blocks;
         ctx->trace_blocks_per_sm = c.per_sm;
         ctx->trace_order = c.order;
-        ctx->trace_node_test = c.node_test;
         cudaError_t e = launch_trace(ctx, rays, n, any_hit, ctx->stage_out.ptr, ctx->stream);  // warm-up
         float ms = 0.0f, total = 0.0f;
         for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
@@ -645,7 +531,6 @@ rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
             ctx->trace_min_blocks = saved.min_blocks;
             ctx->trace_blocks_per_sm = saved.per_sm;
             ctx->trace_order = saved.order;
-            ctx->trace_node_test = saved.node_test;
             return cuda_fail(ctx, e, "autotune launch");
         }
         if (total < best_ms) {
@@ -659,7 +544,6 @@ rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
     ctx->trace_min_blocks = best.min_blocks;
     ctx->trace_blocks_per_sm = best.per_sm;
     ctx->trace_order = best.order;
-    ctx->trace_node_test = best.node_test;
     if (chosen_ms_x1000) *chosen_ms_x1000 = static_cast<int64_t>(best_ms / 3.0f * 1000.0f);
     return check_device_error(ctx, ctx->stream);
 }
