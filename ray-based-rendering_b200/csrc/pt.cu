@@ -35,24 +35,25 @@ constexpr int kLoopScenes = 16;  // scenes one persistent batched run can addres
 constexpr uint32_t kDefaultCapacity = 1u << 22;  // most samples per pixel in one call (a wave holds a pixel's samples)
 constexpr size_t kShadowBytesLimit = size_t(2) << 30;
 
-// counters (uint32 words)
+// Counters (uint32 words). The ones that many warps update at once (queue counts, claim cursors)
+// lie on 128-byte lines of their own: the L2 serves the atomics of one line one after another, so
+// cursors and counts that share a line wait for each other.
+constexpr int kLine = 32;
 enum : int {
-    kCQ0 = 0,       // active queue counts, ping-pong by depth parity
-    kCClass = 2,    // kNumClasses class-queue counts
-    kCShadow = 8,   // shadow queue count
-    kCExt = 10,     // 64-bit: extension rays traced
-    kCSh = 12,      // 64-bit: shadow rays traced
-    kCQuery = 14,   // radiance cache: paths ended into the cache in this wave
-    kCTrain = 15,   // radiance cache: training vertices gathered in this frame
-    kCTrainBase = 16,  // radiance cache: kCTrain at the start of this wave
-    kCShade = 18,      // 64-bit: hit vertices shaded
-    kCTraffic = 20,    // 4 x 64-bit (RBR_RENDER_COUNT_TRAFFIC): extension nodes, records; shadow nodes, records
-    kCCursor = 28,     // 3 claim cursors of one depth (Paths::fetch): extension, shading, shadow queue
-    kCWords = 32
+    kCQ0 = 0,                // active queue counts, ping-pong by depth parity
+    kCClass = kLine,         // kNumClasses class-queue counts, a line each
+    kCShadow = kCClass + static_cast<int>(kNumClasses) * kLine,  // shadow queue count
+    kCCursor = kCShadow + kLine,  // 3 claim cursors of one depth (Paths::fetch): extension, shading, shadow queue
+    kCQuery = kCCursor + 3 * kLine,  // radiance cache: paths ended into the cache in this wave
+    kCTrain = kCQuery + kLine,       // radiance cache: training vertices gathered in this frame
+    kCTrainBase = kCTrain + 1,       // radiance cache: kCTrain at the start of this wave
+    kCExt = kCTrain + kLine,         // 64-bit: extension rays traced
+    kCSh = kCExt + 2,                // 64-bit: shadow rays traced
+    kCShade = kCSh + 2,              // 64-bit: hit vertices shaded
+    kCTraffic = kCShade + 2,         // 4 x 64-bit (RBR_RENDER_COUNT_TRAFFIC): extension nodes, records; shadow nodes, records
+    kCWords = kCExt + kLine
 };
-static_assert(kCClass + static_cast<int>(kNumClasses) <= kCShadow, "class-queue counts overlap the shadow count");
-static_assert(kCExt % 2 == 0 && kCSh % 2 == 0 && kCShade % 2 == 0 && kCTraffic % 2 == 0, "64-bit counters");
-static_assert(kCTraffic + 8 <= kCCursor && kCCursor + 3 <= kCWords, "claim cursors overlap");
+static_assert(kCExt % 2 == 0 && kCTraffic + 8 <= kCWords, "64-bit counters");
 
 // The blocks a stage runs on: the whole grid for the wavefront kernels, one half of it for a
 // half of the persistent wave loop. Grid-stride loops start at block `block` of `blocks`.
@@ -273,13 +274,12 @@ __global__ void __launch_bounds__(kBlock) k_raygen(CameraDev cam, Wave w, Paths 
     raygen_body<kPacked>(cam, w, P, grid_span());
 }
 
-// Resets the counters depth `d` appends to.
+// Resets the counters depth `d` appends to (called by one warp).
 __device__ __forceinline__ void begin_body(const Paths& P, uint32_t d) {
-    uint32_t* c = P.counters;
-    c[kCQ0 + ((d + 1) & 1)] = 0;
-    for (int i = 0; i < kNumClasses; ++i) c[kCClass + i] = 0;
-    c[kCShadow] = 0;
-    for (int i = 0; i < 3; ++i) c[kCCursor + i] = 0;
+    constexpr uint32_t kCounts = kNumClasses + 1 + 3;  // classes, shadow queue, cursors: consecutive lines
+    static_assert(kCCursor + 3 * kLine == kCClass + static_cast<int>(kCounts) * kLine, "one run of lines");
+    if (threadIdx.x < kCounts) P.counters[kCClass + threadIdx.x * kLine] = 0;
+    if (threadIdx.x == kCounts) P.counters[kCQ0 + ((d + 1) & 1)] = 0;
 }
 
 __global__ void k_begin(Paths P, uint32_t d) {
@@ -357,7 +357,7 @@ __device__ __forceinline__ void extend_body(const DeviceScene& s, const Wave& w,
             const int leader = __ffs(peers) - 1;
             uint32_t first = 0;
             if (cls < kNumClasses && static_cast<int>(threadIdx.x & 31) == leader)
-                first = atomicAdd(P.counters + kCClass + cls, __popc(peers));
+                first = atomicAdd(P.counters + kCClass + cls * kLine, __popc(peers));
             first = __shfl_sync(0xFFFFFFFFu, first, leader);
             if (cls < kNumClasses) P.classq[cls * P.cap + first + __popc(peers & lanemask_lt())] = k;
         }
@@ -521,13 +521,13 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
     uint32_t cnt[kNumClasses + 1];
     cnt[0] = 0;
     if (kCls < 0)
-        for (int c = 0; c < kNumClasses; ++c) cnt[c + 1] = cnt[c] + P.counters[kCClass + c];
-    const uint32_t n = kCls < 0 ? cnt[kNumClasses] : P.counters[kCClass + (kCls < 0 ? 0 : kCls)];
+        for (int c = 0; c < kNumClasses; ++c) cnt[c + 1] = cnt[c] + P.counters[kCClass + c * kLine];
+    const uint32_t n = kCls < 0 ? cnt[kNumClasses] : P.counters[kCClass + (kCls < 0 ? 0 : kCls) * kLine];
     uint32_t* nextq = (d & 1) ? P.q0 : P.q1;
     uint32_t* nextc = P.counters + kCQ0 + ((d + 1) & 1);
     if (g.block == 0 && threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(P.counters + kCShade), n);
     // one cursor per depth: the per-class launches keep the grid-stride order
-    Claim cl(P.fetch && kCls < 0 ? P.counters + kCCursor + 1 : nullptr, n, g);
+    Claim cl(P.fetch && kCls < 0 ? P.counters + kCCursor + kLine : nullptr, n, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
         const bool valid = j < n;
         uint32_t k = 0;
@@ -706,7 +706,7 @@ __device__ __forceinline__ void shadow_body(const DeviceScene& s, const Paths& P
     }
     if (g.block == 0 && threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(P.counters + kCSh), n);
     uint2 traffic = make_uint2(0u, 0u);
-    Claim cl(P.fetch ? P.counters + kCCursor + 2 : nullptr, n, g);
+    Claim cl(P.fetch ? P.counters + kCCursor + 2 * kLine : nullptr, n, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
         if (j < n) {  // lanes past the end claim again with their warp
             const float4* e = P.shadow + 3 * static_cast<size_t>(j);
@@ -904,7 +904,7 @@ __global__ void __launch_bounds__(kBlock, 8) k_wave_loop(const __grid_constant__
         loop_raygen(P, g);
         if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
         for (uint32_t d = 0; d < lw.max_depth; ++d) {
-            if (g.block == 0 && threadIdx.x == 0) begin_body(P, d);
+            if (g.block == 0 && threadIdx.x < 32) begin_body(P, d);
             if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
             if (lw.mode == 2) loop_extend<true>(s, P, d, p.err, g);
             else loop_extend<false>(s, P, d, p.err, g);
@@ -1098,7 +1098,7 @@ rbr_status render(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_params* 
         k_raygen<false><<<grid, kBlock, 0, ws>>>(cd, w, P);
         ++launches;
         for (uint32_t d = 0; d < w.max_depth; ++d) {
-            k_begin<<<1, 1, 0, ws>>>(P, d);
+            k_begin<<<1, 32, 0, ws>>>(P, d);
             if (volumetric) {
                 if (count) k_extend<true, false, true><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
                 else k_extend<true, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
@@ -1286,7 +1286,7 @@ rbr_status render_cached(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_p
             k_raygen<false><<<grid, kBlock, 0, ws>>>(cd, w, P);
             ++launches;
             for (uint32_t d = 0; d < w.max_depth; ++d) {
-                k_begin<<<1, 1, 0, ws>>>(P, d);
+                k_begin<<<1, 32, 0, ws>>>(P, d);
                 k_extend<false, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
                 k_shade<1, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
                 k_shadow<<<grid, kBlock, 0, ws>>>(ctx->scene, P, ctx->d_error);
@@ -1387,7 +1387,7 @@ cudaError_t launch_packed_wave(rbr_ctx* eng, rbr_ctx* scn, const PackedWave& pw,
     if (e != cudaSuccess) return e;
     k_raygen<true><<<grid, kBlock, 0, stream>>>(unused, w, P);
     for (uint32_t d = 0; d < pw.max_depth; ++d) {
-        k_begin<<<1, 1, 0, stream>>>(P, d);
+        k_begin<<<1, 32, 0, stream>>>(P, d);
         if (pw.mode == 2) {
             k_extend<true, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d, eng->d_error);
             k_shade<2, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d);
@@ -1517,7 +1517,7 @@ rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_
     // per light and path
     const uint32_t nl = std::max(1u, ctx->scene.num_lights);
     const size_t per_path = 88 + 4 * size_t(kNumClasses) + 48 * size_t(nl);
-    const size_t fixed = 9 * 256;  // counters + alignment of the eight arrays
+    const size_t fixed = align256(kCWords * 4) + 8 * 256;  // counters + alignment of the eight arrays
     uint64_t cap = (RBR_NOALLOC_SCRATCH_BYTES - fixed) / per_path;
     cap = std::min<uint64_t>(cap, npix * spp);
     cap = cap / spp * spp;
@@ -1587,7 +1587,7 @@ rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_
         w.seed = p->seed;
         k_raygen<false><<<grid, kBlock, 0, stream>>>(cd, w, P);
         for (uint32_t d = 0; d < w.max_depth; ++d) {
-            k_begin<<<1, 1, 0, stream>>>(P, d);
+            k_begin<<<1, 32, 0, stream>>>(P, d);
             k_extend<false, false><<<grid, kBlock, 0, stream>>>(ctx->scene, w, P, d, ctx->d_error);
             k_shade<0, false><<<grid, kBlock, 0, stream>>>(ctx->scene, w, P, d);
             k_shadow<<<grid, kBlock, 0, stream>>>(ctx->scene, P, ctx->d_error);
