@@ -239,13 +239,16 @@ rbr_status rbr_scene_upload(rbr_ctx* ctx, const rbr_scene_desc* desc);
 rbr_status rbr_scene_stats_get(const rbr_ctx* ctx, rbr_scene_stats* out);
 
 /* Tunables of a context (no reference counterpart). Names:
- *   "trace.kernel"         0: one thread per ray (default); 1: persistent warps that hand a
- *                          finished lane the next ray of the warp's chunk; 2: warp-cooperative,
- *                          8 lanes per ray, one child box per lane
+ *   "trace.kernel"         0 (default): persistent warps that trace coherent rays one thread per
+ *                          ray and others by warp traversal (a finished lane takes the next ray,
+ *                          leaf records are shared out over the warp), each warp by its own rays;
+ *                          one thread per ray where "trace.order" sorts them; 1: warp traversal
+ *                          always; 2: warp-cooperative, 8 lanes per ray, one child box per lane
  *   "trace.blocks_per_sm"  resident blocks per SM of kernels 1 and 2 (0: occupancy limit)
  *   "trace.refill_min"     kernel 1: idle lanes a warp waits for before it fetches new rays,
  *                          1..32 (default 1: refill after every step with an idle lane)
- *   "trace.min_blocks"     kernel 0's register budget: 8, 10 or 12 resident blocks per SM
+ *   "trace.min_blocks"     kernel 0 on sorted rays: register budget for 8, 10 or 12 resident
+ *                          blocks per SM
  *   "trace.order"          kernels 0 and 1: 0 traces the rays in the order given; 1..5 first sort
  *                          them on the device so that warps hold rays that walk the same nodes:
  *                          1 by direction octant, then origin cell of 512^3; 2 octant, then cell
@@ -295,7 +298,7 @@ rbr_status rbr_scene_stats_get(const rbr_ctx* ctx, rbr_scene_stats* out);
 rbr_status rbr_param_set(rbr_ctx* ctx, const char* name, int64_t value);
 rbr_status rbr_param_get(const rbr_ctx* ctx, const char* name, int64_t* value);
 /* Autotuner (no reference counterpart): times the traversal variants ("trace.kernel",
- * "trace.min_blocks", "trace.order" 0, 4 and 5) on n rays of the caller's own
+ * "trace.min_blocks", "trace.order" 0, 4 and 5, "trace.refill_min") on n rays of the caller's own
  * workload (device pointer) against the uploaded scene, keeps the fastest in the context and
  * returns its time per launch in microseconds (out_us may be NULL). Waits for the timings. */
 rbr_status rbr_autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, int64_t* out_us);

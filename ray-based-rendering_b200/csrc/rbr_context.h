@@ -57,9 +57,9 @@ struct rbr_ctx {
     uint32_t* d_cursors = nullptr;
     uint32_t cursor_next = 0;
     // tunables (rbr_param_set / rbr_autotune)
-    int trace_kernel = 0;          // 0: one thread per ray, 1: persistent lane refill, 2: warp-cooperative
+    int trace_kernel = 0;          // 0: adaptive persistent warps, 1: warp traversal with lane refill, 2: warp-cooperative
     int trace_blocks_per_sm = 0;   // persistent grid per SM (0: occupancy limit)
-    int trace_min_blocks = 10;     // kernel 0: register budget for 8, 10 or 12 resident blocks per SM
+    int trace_min_blocks = 10;     // kernel 0 on sorted rays: register budget for 8, 10 or 12 resident blocks per SM
     int trace_order = 0;           // kernel 0: 0 rays in the given order, 1 sorted by direction octant and origin
     int trace_node_test = 0;       // accepted and reported, without effect (one node test)
     int trace_stream_io = 1;       // kernel 0: rays read and hits written with evict-first (streaming) hints
@@ -137,16 +137,8 @@ rbr_status upload_scene_variant(rbr_ctx* dst, const rbr_ctx* base, const rbr_mat
 void free_scene(rbr_ctx* ctx);
 
 // kernels (trace.cu)
-cudaError_t launch_trace_closest(const DeviceScene& s, const rbr_ray* rays, uint32_t n, rbr_hit* hits, int* err,
-                                 int num_sms, cudaStream_t stream);
-cudaError_t launch_trace_any(const DeviceScene& s, const rbr_ray* rays, uint32_t n, uint8_t* occ, int* err,
-                             int num_sms, cudaStream_t stream);
 cudaError_t launch_trace_counts(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit,
                                 unsigned long long* totals, int* err, cudaStream_t stream);
-cudaError_t launch_trace_persist(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit, void* out,
-                                 int* err, uint32_t* cursor, int grid, cudaStream_t stream, const uint32_t* perm = nullptr,
-                                 uint32_t refill_min = 1);
-int trace_persist_blocks_per_sm(int any_hit);
 cudaError_t launch_trace_coop(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit, void* out, int* err,
                               uint32_t* cursor, int grid, cudaStream_t stream);
 int trace_coop_blocks_per_sm(int any_hit);

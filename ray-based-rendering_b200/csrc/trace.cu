@@ -1,6 +1,6 @@
 // Ray-query kernels: closest hit and any hit for a batch of rbr_ray records.
 //
-// One thread per ray. Rays are read as two 16 B words (origin+tmax, direction+pad), answers
+// Rays are read as two 16 B words (origin+tmax, direction+pad), answers
 // written as one 8 B word (closest) or one byte (any). The traversal itself is in
 // rbr_device.cuh.
 #include <algorithm>
@@ -28,23 +28,11 @@ __device__ __forceinline__ void put_hit(uint2* p, uint2 h) {
     else *p = h;
 }
 
-// kMinBlocks: resident blocks per SM the register allocation must allow (8: up to 64
-// registers a thread, 10: 48, 12: 40) -- occupancy against register spills, picked by tuning.
-template <int kMinBlocks, bool kStream>
-__global__ void __launch_bounds__(kTraceBlock, kMinBlocks) k_trace_closest(DeviceScene s, const float4* __restrict__ rays,
-                                                                           uint32_t n, uint2* __restrict__ hits, int* err) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 a = ray_word<kStream>(rays + 2 * static_cast<size_t>(i));
-    const float4 b = ray_word<kStream>(rays + 2 * static_cast<size_t>(i) + 1);
-    float t = 0.0f;
-    const uint32_t prim = traverse<false>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, t, err);
-    put_hit<kStream>(hits + i, make_uint2(prim, prim == 0xFFFFFFFFu ? 0u : __float_as_uint(t)));
-}
-
-// The same query on the rays in the order `perm` (a permutation of 0..n-1): rays that start
-// close together with directions of the same octant share warps, so they walk the same nodes.
-// Answers go to the rays' own positions.
+// One thread per ray in the order `perm` (a permutation of 0..n-1): rays that start close together
+// with directions of the same octant share warps, so they walk the same nodes. Answers go to the
+// rays' own positions. kMinBlocks: resident blocks per SM the register allocation must allow (8:
+// up to 64 registers a thread, 10: 48, 12: 40) -- occupancy against register spills, picked by
+// tuning.
 template <int kMinBlocks, bool kStream>
 __global__ void __launch_bounds__(kTraceBlock, kMinBlocks)
     k_trace_closest_perm(DeviceScene s, const float4* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ perm,
@@ -178,16 +166,6 @@ __global__ void k_ray_scatter16(const uint16_t* __restrict__ keys, uint32_t n, u
     scatter_keys<kScanChunks>(keys, n, offsets, chunk_sum, perm);
 }
 
-__global__ void __launch_bounds__(kTraceBlock) k_trace_any(DeviceScene s, const float4* __restrict__ rays, uint32_t n,
-                                                           uint8_t* __restrict__ occ, int* err) {
-    const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 a = __ldg(rays + 2 * static_cast<size_t>(i));
-    const float4 b = __ldg(rays + 2 * static_cast<size_t>(i) + 1);
-    float t;
-    occ[i] = static_cast<uint8_t>(traverse<true>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, t, err));
-}
-
 // Same traversal, counting wide nodes fetched and leaf records tested (summed over the batch).
 template <bool kAny>
 __global__ void __launch_bounds__(kTraceBlock) k_trace_count(DeviceScene s, const float4* __restrict__ rays,
@@ -217,71 +195,142 @@ __device__ __forceinline__ uint32_t lane_mask_lt() {
     return m;
 }
 
-// The answer of a finished TraceState for ray idx.
-template <bool kAny>
-__device__ __forceinline__ void put_answer(uint2* hits, uint8_t* occ, uint32_t idx, const TraceState& st, uint32_t anyhit) {
-    if (kAny) occ[idx] = static_cast<uint8_t>(anyhit);
-    else hits[idx] = make_uint2(st.best < 0 ? 0xFFFFFFFFu : static_cast<uint32_t>(st.best),
-                                st.best < 0 ? 0u : __float_as_uint(st.tbest));
+// Persistent warps: each warp starts with the 32 rays of its own index and claims the next 32 from
+// a global cursor when it needs more. Incoherent rays were bound by instruction issue at 8 to 12 of
+// 32 lanes active: some rays of a warp end long before others, and few lanes test leaf records at
+// once. A warp looks at its first rays and keeps to one of two ways:
+//   - Warp traversal (rbr_device.cuh), and the next rays go to lanes whose ray is done while the
+//     others are still traversing: 29 of 32 lanes busy in the node test, one round of record tests
+//     a step. 2^22 uniform rays through 1.3M triangles 1,620 -> 1,068 us (sorted first, one thread
+//     per ray: 1,380), any hit 1,240 -> 871; 2^22 shadow segments over 2M triangles 838 -> 501;
+//     1,024 to 2^16 rays, bound by the longest traversals, unchanged to 20 % faster.
+//   - Coherent rays (neighbouring origins, nearly the same direction: camera rays in scanline
+//     order) walk the same nodes and finish together: one thread per ray, 32 new rays when all are
+//     done, where coherent_pays().
+// A claim is 32 rays whatever the batch: with claims of up to 256 the warps that drew the long
+// traversals of a camera image kept a launch alive behind the others (2^22 rays 1,701 us, 764 at
+// 32). Not kept: claiming the next run ahead of a traversal (679 us instead of 591: a held run
+// waits behind a long one), records tested by their own lane where many lanes have one.
+// With `perm` (sorted rays), position j of the order is ray perm[j]. kRefillOnly: every warp goes
+// the second way.
+constexpr int kPersistBlock = 128;
+constexpr uint32_t kClaimRays = 32;
+constexpr uint32_t kAdaptiveRefill = 6;  // idle lanes before a refill (4 to 8 measured within 2 %)
+
+// Origins within 1/16 of the tree's extent of the warp's first ray's and directions within 11
+// degrees of its: half of a 32-ray run of camera rays spans a degree, rays after a bounce the
+// sphere. The choice changes no answer.
+__device__ __forceinline__ bool coherent_rays(const DeviceScene& s, bool valid, float4 a, float4 b) {
+    const float ox = __shfl_sync(0xFFFFFFFFu, a.x, 0), oy = __shfl_sync(0xFFFFFFFFu, a.y, 0), oz = __shfl_sync(0xFFFFFFFFu, a.z, 0);
+    const float dx = __shfl_sync(0xFFFFFFFFu, b.x, 0), dy = __shfl_sync(0xFFFFFFFFu, b.y, 0), dz = __shfl_sync(0xFFFFFFFFu, b.z, 0);
+    const float off = fabsf(a.x - ox) + fabsf(a.y - oy) + fabsf(a.z - oz);
+    const float c = b.x * dx + b.y * dy + b.z * dz;
+    const float l2 = (b.x * b.x + b.y * b.y + b.z * b.z) * (dx * dx + dy * dy + dz * dz);
+    const bool near = off <= 0.125f * s.tree_reach && c > 0.0f && c * c >= 0.9635f * l2;
+    return __all_sync(0xFFFFFFFFu, !valid || near);
 }
 
-// Persistent warps: each warp takes chunks of kChunk consecutive rays from a global cursor
-// (one atomic per chunk) and hands the next ray of its chunk to any lane whose ray is done,
-// so lanes keep working while the warp's other rays are still traversing. Every loop
-// iteration each active lane advances its ray by one step (a leaf-record test or a node test).
-// With `perm` (sorted rays), position j of the cursor's order is ray perm[j].
-constexpr int kPersistBlock = 128;
-constexpr uint32_t kChunk = 256;
+// Whether one thread per ray pays for coherent rays: where most of a launch is throughput, not the
+// latency of its longest traversals. Camera rays, one thread per ray against warp traversal (us):
+// Cornell box, 2^18 rays 27 / 31, 2^22 131 / 202; 20 K triangles 2^20 121 / 123, 2^21 174 / 198;
+// 405 K 2^20 222 / 191, 2^21 275 / 270, 2^22 390 / 428; 2 M 2^21 437 / 370, 2^22 589 / 540.
+__device__ __forceinline__ bool coherent_pays(const DeviceScene& s, uint32_t n) {
+    return n / 32u >= s.num_nodes && (n >= (1u << 20) || s.num_nodes <= 64u);
+}
 
-template <bool kAny>
-__global__ void __launch_bounds__(kPersistBlock) k_trace_persist(DeviceScene s, const float4* __restrict__ rays,
-                                                                 uint32_t n, const uint32_t* __restrict__ perm,
-                                                                 uint2* __restrict__ hits, uint8_t* __restrict__ occ,
-                                                                 int* err, uint32_t* cursor, uint32_t refill_min) {
+template <bool kAny, bool kStream, bool kRefillOnly>
+__global__ void __launch_bounds__(kPersistBlock, 8)
+    k_trace(DeviceScene s, const float4* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ perm,
+            uint2* __restrict__ hits, uint8_t* __restrict__ occ, int* err, uint32_t* cursor, uint32_t refill_min) {
+    __shared__ WarpRays shared[kPersistBlock / 32];
+    WarpRays& w = shared[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
-    uint32_t chunk_next = 0, chunk_end = 0;  // warp-uniform
-    bool exhausted = false;                  // warp-uniform
-    uint32_t idx = 0xFFFFFFFFu;              // this lane's ray
-    uint32_t anyhit = 0;
-    TraceState st;
+    const uint32_t first = gridDim.x * kPersistBlock;  // rays before this belong to the warps' first runs
+    uint32_t run = blockIdx.x * kPersistBlock + (threadIdx.x & ~31u);  // warp-uniform
+    if (run >= n) return;
+    uint32_t end = run + min(kClaimRays, n - run);  // warp-uniform
+    // the warp's next run of rays; false when there is none (the cursor is unused, and need not be
+    // reset, while every ray is in a first run)
+    auto claim = [&]() {
+        if (n <= first) return false;
+        uint32_t b = 0;
+        if (lane == 0) b = atomicAdd(cursor, kClaimRays);
+        run = first + __shfl_sync(0xFFFFFFFFu, b, 0);
+        if (run < first || run >= n) return false;  // past the end (run < first: past 2^32)
+        end = run + min(kClaimRays, n - run);
+        return true;
+    };
+    if (!kRefillOnly && coherent_pays(s, n)) {
+        uint32_t i = run + lane;
+        bool valid = i < end;
+        float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
+        if (valid) {
+            a = ray_word<kStream>(rays + 2 * static_cast<size_t>(i));
+            b = ray_word<kStream>(rays + 2 * static_cast<size_t>(i) + 1);
+        }
+        if (coherent_rays(s, valid, a, b)) {
+            while (true) {
+                if (valid) {
+                    float t = 0.0f;
+                    const uint32_t r = traverse<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, t, err);
+                    if (kAny) occ[i] = static_cast<uint8_t>(r);
+                    else put_hit<kStream>(hits + i, make_uint2(r, r == 0xFFFFFFFFu ? 0u : __float_as_uint(t)));
+                }
+                if (!claim()) return;
+                i = run + lane;
+                valid = i < end;
+                if (valid) {
+                    a = ray_word<kStream>(rays + 2 * static_cast<size_t>(i));
+                    b = ray_word<kStream>(rays + 2 * static_cast<size_t>(i) + 1);
+                }
+            }
+        }
+    }
+    bool exhausted = false;      // warp-uniform
+    uint32_t idx = 0xFFFFFFFFu;  // this lane's ray
+    LaneRay lr;
     uint2 stack[kStackSize];
+    auto answer = [&]() {
+        const unsigned long long b = w.best[lane];
+        if (kAny) {
+            occ[idx] = b != 0;
+        } else {
+            const uint32_t prim = hit_prim(b);
+            put_hit<kStream>(hits + idx, make_uint2(prim, prim == 0xFFFFFFFFu ? 0u : hit_tbits(b)));
+        }
+        idx = 0xFFFFFFFFu;
+    };
     while (true) {
         uint32_t need = __ballot_sync(0xFFFFFFFFu, idx == 0xFFFFFFFFu);
         // refill once at least refill_min lanes are idle (or all of them): a refill costs the
         // whole warp a few ballots and a ray load, so lanes may idle for a few steps first
         while (need != 0 && !exhausted && (static_cast<uint32_t>(__popc(need)) >= refill_min || need == 0xFFFFFFFFu)) {
-            if (chunk_next == chunk_end) {
-                uint32_t b = 0;
-                if (lane == 0) b = atomicAdd(cursor, kChunk);
-                b = __shfl_sync(0xFFFFFFFFu, b, 0);
-                if (b >= n) {
-                    exhausted = true;
-                    break;
-                }
-                chunk_next = b;
-                chunk_end = min(b + kChunk, n);
+            if (run >= end && !claim()) {
+                exhausted = true;
+                break;
             }
-            const uint32_t avail = chunk_end - chunk_next;
-            const uint32_t rank = __popc(need & lane_mask_lt());
-            if (((need >> lane) & 1u) && rank < avail) {
-                idx = perm ? __ldg(perm + chunk_next + rank) : chunk_next + rank;
-                const float4 a = __ldg(rays + 2 * static_cast<size_t>(idx));
-                const float4 b = __ldg(rays + 2 * static_cast<size_t>(idx) + 1);
-                if (trace_begin<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, st, anyhit)) {
-                    put_answer<kAny>(hits, occ, idx, st, anyhit);
-                    idx = 0xFFFFFFFFu;  // finished at once: takes another ray in this round
-                }
+            const uint32_t j = run + __popc(need & lane_mask_lt());
+            if (((need >> lane) & 1u) && j < end) {
+                idx = perm ? __ldg(perm + j) : j;
+                const float4 a = ray_word<kStream>(rays + 2 * static_cast<size_t>(idx));
+                const float4 b = ray_word<kStream>(rays + 2 * static_cast<size_t>(idx) + 1);
+                // finished at once: takes another ray in this round
+                if (lane_begin<kAny>(s, w, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, lr)) answer();
             }
-            chunk_next += min(__popc(need), avail);  // each round consumes at least one ray
+            run = min(end, run + __popc(need));  // each round consumes at least one ray
             need = __ballot_sync(0xFFFFFFFFu, idx == 0xFFFFFFFFu);
         }
         const bool active = idx != 0xFFFFFFFFu;
         if (__ballot_sync(0xFFFFFFFFu, active) == 0) break;  // only when the rays are exhausted
-        if (active && trace_step<kAny>(s, st, stack, err, anyhit)) {
-            put_answer<kAny>(hits, occ, idx, st, anyhit);
-            idx = 0xFFFFFFFFu;
-        }
+        if (warp_step<kAny>(s, w, active, lr, stack, err)) answer();
     }
+}
+
+// The warp's next claim of `count` rays from position x on; x >= n when the rays are exhausted.
+__device__ __forceinline__ uint32_t claim_rays(uint32_t* cursor, uint32_t count) {
+    uint32_t b = 0;
+    if ((threadIdx.x & 31u) == 0) b = atomicAdd(cursor, count);
+    return __shfl_sync(0xFFFFFFFFu, b, 0);
 }
 
 // ------------------------------------------------------------------------------------------
@@ -294,28 +343,34 @@ template <bool kAny>
 __global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const float4* __restrict__ rays, uint32_t n,
                                                            uint2* __restrict__ hits, uint8_t* __restrict__ occ,
                                                            int* err, uint32_t* cursor) {
-    const uint32_t lane = threadIdx.x & 31u;
     const GroupLanes g = group_lanes();
+    // an equal share for every warp, at least the four rays it traces at once
+    const uint32_t claim = min(32u, max(4u, n / (gridDim.x * (kCoopBlock / 32))));
     uint32_t chunk_next = 0, chunk_end = 0;   // warp-uniform
     bool exhausted = false;                   // warp-uniform
     uint32_t idx = 0xFFFFFFFFu;               // group-uniform
     uint32_t anyhit = 0;
-    TraceState st{};
+    GroupRay st{};
     uint2 stack[kStackSize];
+    auto answer = [&]() {
+        if (g.j == 0) {
+            if (kAny) occ[idx] = static_cast<uint8_t>(anyhit);
+            else hits[idx] = make_uint2(st.best < 0 ? 0xFFFFFFFFu : static_cast<uint32_t>(st.best),
+                                        st.best < 0 ? 0u : __float_as_uint(st.tbest));
+        }
+        idx = 0xFFFFFFFFu;
+    };
     while (true) {
         // give idle groups new rays from the warp's chunk
         uint32_t need = __ballot_sync(0xFFFFFFFFu, g.j == 0 && idx == 0xFFFFFFFFu);
         while (need != 0 && !exhausted) {
             if (chunk_next == chunk_end) {
-                uint32_t b = 0;
-                if (lane == 0) b = atomicAdd(cursor, kChunk);
-                b = __shfl_sync(0xFFFFFFFFu, b, 0);
-                if (b >= n) {
+                chunk_next = claim_rays(cursor, claim);
+                if (chunk_next >= n) {
                     exhausted = true;
                     break;
                 }
-                chunk_next = b;
-                chunk_end = min(b + kChunk, n);
+                chunk_end = min(chunk_next + claim, n);
             }
             const uint32_t avail = chunk_end - chunk_next;
             const uint32_t rank = __popc(need & ((1u << g.shift) - 1u));
@@ -323,19 +378,14 @@ __global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const 
                 idx = chunk_next + rank;
                 const float4 a = __ldg(rays + 2 * static_cast<size_t>(idx));
                 const float4 b = __ldg(rays + 2 * static_cast<size_t>(idx) + 1);
-                if (trace_begin<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, st, anyhit)) {
-                    if (g.j == 0) put_answer<kAny>(hits, occ, idx, st, anyhit);
-                    idx = 0xFFFFFFFFu;  // finished at once: takes another ray in this round
-                }
+                // finished at once: takes another ray in this round
+                if (group_begin<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, st, anyhit)) answer();
             }
             chunk_next += min(__popc(need), avail);
             need = __ballot_sync(0xFFFFFFFFu, g.j == 0 && idx == 0xFFFFFFFFu);
         }
         if (__ballot_sync(0xFFFFFFFFu, idx != 0xFFFFFFFFu) == 0) break;  // rays exhausted
-        if (idx != 0xFFFFFFFFu && group_step<kAny>(s, g, st, stack, err, anyhit)) {
-            if (g.j == 0) put_answer<kAny>(hits, occ, idx, st, anyhit);
-            idx = 0xFFFFFFFFu;
-        }
+        if (idx != 0xFFFFFFFFu && group_step<kAny>(s, g, st, stack, err, anyhit)) answer();
     }
 }
 
@@ -361,20 +411,32 @@ int trace_coop_blocks_per_sm(int any_hit) {
     return b > 0 ? b : 1;
 }
 
-cudaError_t launch_trace_persist(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit, void* out,
-                                 int* err, uint32_t* cursor, int grid, cudaStream_t stream, const uint32_t* perm,
-                                 uint32_t refill_min) {
-    if (n == 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(uint32_t), stream);
-    if (e != cudaSuccess) return e;
-    const auto* r = reinterpret_cast<const float4*>(rays);
-    if (any_hit)
-        k_trace_persist<true><<<grid, kPersistBlock, 0, stream>>>(s, r, n, perm, nullptr, static_cast<uint8_t*>(out),
-                                                                  err, cursor, refill_min);
-    else
-        k_trace_persist<false><<<grid, kPersistBlock, 0, stream>>>(s, r, n, perm, static_cast<uint2*>(out), nullptr,
-                                                                   err, cursor, refill_min);
-    return cudaGetLastError();
+// Kernels 0 (in the given order) and 1: k_trace with the context's parameters.
+static cudaError_t launch_trace_warps(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, void* out,
+                                      const uint32_t* perm, cudaStream_t stream) {
+    const bool refill_only = ctx->trace_kernel == 1;
+    const bool st = ctx->trace_stream_io != 0;
+    auto k = any_hit ? (refill_only ? (st ? k_trace<true, true, true> : k_trace<true, false, true>)
+                                    : (st ? k_trace<true, true, false> : k_trace<true, false, false>))
+                     : (refill_only ? (st ? k_trace<false, true, true> : k_trace<false, false, true>)
+                                    : (st ? k_trace<false, true, false> : k_trace<false, false, false>));
+    int per_sm = refill_only ? ctx->trace_blocks_per_sm : 0;
+    if (per_sm == 0) {
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k, kPersistBlock, 0);
+        if (e != cudaSuccess) return e;
+        per_sm = std::max(1, per_sm);
+    }
+    // no more warps than there are runs of rays
+    const uint32_t grid = static_cast<uint32_t>(std::max<uint64_t>(
+        1, std::min<uint64_t>(uint64_t(ctx->num_sms) * per_sm, (uint64_t(n) + kPersistBlock - 1) / kPersistBlock)));
+    uint32_t* cursor = ctx->d_cursors + (ctx->cursor_next++ % kCursorRing);
+    if (n > grid * kPersistBlock) {
+        cudaError_t e = cudaMemsetAsync(cursor, 0, sizeof(uint32_t), stream);
+        if (e != cudaSuccess) return e;
+    }
+    return launch_query(ctx, k, grid, stream, ctx->scene, reinterpret_cast<const float4*>(rays), n, perm,
+                        any_hit ? nullptr : static_cast<uint2*>(out), any_hit ? static_cast<uint8_t*>(out) : nullptr,
+                        ctx->d_error, cursor, refill_only ? static_cast<uint32_t>(ctx->trace_refill_min) : kAdaptiveRefill);
 }
 
 // The sort buffers of the streams of a chunked rbr_trace_host (slot 0: the context's stream).
@@ -458,52 +520,40 @@ cudaError_t launch_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_
         }
         return cudaGetLastError();
     }
-    if (ctx->trace_kernel == 0) {
-        if (any_hit)
-            return launch_trace_any(ctx->scene, rays, n, static_cast<uint8_t*>(out), ctx->d_error, ctx->trace_min_blocks,
-                                    stream);
-        if (n == 0) return cudaSuccess;
-        const uint32_t blocks = (n + kTraceBlock - 1) / kTraceBlock;
-        const auto* r = reinterpret_cast<const float4*>(rays);
-        auto* h = static_cast<uint2*>(out);
-        const bool st = ctx->trace_stream_io != 0;
-        const int mb = ctx->trace_min_blocks;
-        auto k = mb >= 12 ? (st ? k_trace_closest<12, true> : k_trace_closest<12, false>)
-               : mb >= 10 ? (st ? k_trace_closest<10, true> : k_trace_closest<10, false>)
-                          : (st ? k_trace_closest<8, true> : k_trace_closest<8, false>);
-        return launch_query(ctx, k, blocks, stream, ctx->scene, r, n, h, ctx->d_error);
+    if (n == 0) return cudaSuccess;
+    if (ctx->trace_kernel == 2) {
+        const int per_sm = ctx->trace_blocks_per_sm > 0 ? ctx->trace_blocks_per_sm : trace_coop_blocks_per_sm(any_hit);
+        // no more warps than there are groups of 8 lanes to fill
+        const int grid = static_cast<int>(std::max<int64_t>(
+            1, std::min<int64_t>(int64_t(ctx->num_sms) * per_sm, (int64_t(n) + kCoopBlock / 8 - 1) / (kCoopBlock / 8))));
+        uint32_t* cursor = ctx->d_cursors + (ctx->cursor_next++ % kCursorRing);
+        return launch_trace_coop(ctx->scene, rays, n, any_hit, out, ctx->d_error, cursor, grid, stream);
     }
-    const bool coop = ctx->trace_kernel == 2;
     const uint32_t* perm = nullptr;  // kernel 1 refills its lanes in sorted order when trace.order is set
-    if (!coop && ctx->trace_order != 0 && n > 0) {
+    if (ctx->trace_order != 0) {
         cudaError_t e = sort_rays(ctx, sort_slot(ctx, slot), rays, n, &perm, stream);
         if (e != cudaSuccess) return e;
     }
-    const int per_sm = ctx->trace_blocks_per_sm > 0
-                           ? ctx->trace_blocks_per_sm
-                           : (coop ? trace_coop_blocks_per_sm(any_hit) : trace_persist_blocks_per_sm(any_hit));
-    // no more warps than there are chunks of rays
-    const int need = static_cast<int>((n + kChunk - 1) / kChunk + (kPersistBlock / 32) - 1) / (kPersistBlock / 32);
-    const int grid = std::max(1, std::min(ctx->num_sms * per_sm, need));
-    uint32_t* cursor = ctx->d_cursors + (ctx->cursor_next++ % kCursorRing);
-    if (coop) return launch_trace_coop(ctx->scene, rays, n, any_hit, out, ctx->d_error, cursor, grid, stream);
-    return launch_trace_persist(ctx->scene, rays, n, any_hit, out, ctx->d_error, cursor, grid, stream, perm,
-                                static_cast<uint32_t>(ctx->trace_refill_min));
+    return launch_trace_warps(ctx, rays, n, any_hit, out, perm, stream);
 }
 
 // Times every traversal variant on the caller's rays (device pointer) and keeps the fastest.
 rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, int64_t* chosen_ms_x1000) {
     struct Cand {
-        int kernel, min_blocks, per_sm, order;
+        int kernel, min_blocks, per_sm, order, refill;
     };
-    // Unsorted variants, and sorted ones with the 16-bit keys of orders 4 and 5 (the counting
-    // sort of this file). Orders 1-3 (CUB's radix sort) stay selectable by parameter; measured
-    // slower than orders 4 and 5, they are not candidates.
-    const Cand cands[] = {{0, 8, 0, 0}, {0, 10, 0, 0}, {0, 12, 0, 0}, {1, 10, 0, 0}, {2, 10, 0, 0}, {0, 8, 0, 4},
-                          {0, 10, 0, 4}, {0, 12, 0, 4}, {0, 8, 0, 5}, {0, 10, 0, 5}, {0, 12, 0, 5}, {1, 10, 0, 5}};
+    // Rays in the given order (kernel 0 chooses between one thread per ray and warp traversal by
+    // the rays' coherence; kernel 1 always refills), and sorted ones with the 16-bit keys of orders
+    // 4 and 5 (the counting sort of this file). Not candidates: orders 1-3 (CUB's radix sort,
+    // slower than orders 4 and 5) and kernel 2 (slower on batches large enough to tune on); both
+    // stay selectable by parameter.
+    const int refill = ctx->trace_refill_min;
+    const Cand cands[] = {{0, 10, 0, 0, refill}, {1, 10, 0, 0, refill}, {1, 10, 0, 0, 4}, {1, 10, 0, 0, 8},
+                          {0, 8, 0, 4, refill},  {0, 10, 0, 4, refill}, {0, 8, 0, 5, refill}, {0, 10, 0, 5, refill},
+                          {0, 12, 0, 5, refill}, {1, 10, 0, 5, 4}};
     rbr_status st = ensure(ctx, ctx->stage_out, size_t(n) * (any_hit ? 1 : sizeof(rbr_hit)), "autotune output");
     if (st != RBR_OK) return st;
-    const Cand saved{ctx->trace_kernel, ctx->trace_min_blocks, ctx->trace_blocks_per_sm, ctx->trace_order};
+    const Cand saved{ctx->trace_kernel, ctx->trace_min_blocks, ctx->trace_blocks_per_sm, ctx->trace_order, refill};
     float best_ms = 1e30f;
     Cand best = saved;
     cudaEvent_t a, b;
@@ -514,6 +564,7 @@ rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
         ctx->trace_min_blocks = c.min_blocks;
         ctx->trace_blocks_per_sm = c.per_sm;
         ctx->trace_order = c.order;
+        ctx->trace_refill_min = c.refill;
         cudaError_t e = launch_trace(ctx, rays, n, any_hit, ctx->stage_out.ptr, ctx->stream);  // warm-up
         float ms = 0.0f, total = 0.0f;
         for (int k = 0; k < 3 && e == cudaSuccess; ++k) {
@@ -531,6 +582,7 @@ rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
             ctx->trace_min_blocks = saved.min_blocks;
             ctx->trace_blocks_per_sm = saved.per_sm;
             ctx->trace_order = saved.order;
+            ctx->trace_refill_min = saved.refill;
             return cuda_fail(ctx, e, "autotune launch");
         }
         if (total < best_ms) {
@@ -544,15 +596,9 @@ rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
     ctx->trace_min_blocks = best.min_blocks;
     ctx->trace_blocks_per_sm = best.per_sm;
     ctx->trace_order = best.order;
+    ctx->trace_refill_min = best.refill;
     if (chosen_ms_x1000) *chosen_ms_x1000 = static_cast<int64_t>(best_ms / 3.0f * 1000.0f);
     return check_device_error(ctx, ctx->stream);
-}
-
-int trace_persist_blocks_per_sm(int any_hit) {
-    int b = 0;
-    if (any_hit) cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace_persist<true>, kPersistBlock, 0);
-    else cudaOccupancyMaxActiveBlocksPerMultiprocessor(&b, k_trace_persist<false>, kPersistBlock, 0);
-    return b > 0 ? b : 1;
 }
 
 cudaError_t launch_trace_counts(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit,
@@ -563,26 +609,6 @@ cudaError_t launch_trace_counts(const DeviceScene& s, const rbr_ray* rays, uint3
         k_trace_count<true><<<blocks, kTraceBlock, 0, stream>>>(s, reinterpret_cast<const float4*>(rays), n, totals, err);
     else
         k_trace_count<false><<<blocks, kTraceBlock, 0, stream>>>(s, reinterpret_cast<const float4*>(rays), n, totals, err);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_trace_closest(const DeviceScene& s, const rbr_ray* rays, uint32_t n, rbr_hit* hits, int* err,
-                                 int min_blocks, cudaStream_t stream) {
-    if (n == 0) return cudaSuccess;
-    const uint32_t blocks = (n + kTraceBlock - 1) / kTraceBlock;
-    const auto* r = reinterpret_cast<const float4*>(rays);
-    auto* h = reinterpret_cast<uint2*>(hits);
-    if (min_blocks >= 12) k_trace_closest<12, true><<<blocks, kTraceBlock, 0, stream>>>(s, r, n, h, err);
-    else if (min_blocks >= 10) k_trace_closest<10, true><<<blocks, kTraceBlock, 0, stream>>>(s, r, n, h, err);
-    else k_trace_closest<8, true><<<blocks, kTraceBlock, 0, stream>>>(s, r, n, h, err);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_trace_any(const DeviceScene& s, const rbr_ray* rays, uint32_t n, uint8_t* occ, int* err,
-                             int /*num_sms*/, cudaStream_t stream) {
-    if (n == 0) return cudaSuccess;
-    const uint32_t blocks = (n + kTraceBlock - 1) / kTraceBlock;
-    k_trace_any<<<blocks, kTraceBlock, 0, stream>>>(s, reinterpret_cast<const float4*>(rays), n, occ, err);
     return cudaGetLastError();
 }
 
