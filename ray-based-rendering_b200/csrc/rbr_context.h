@@ -139,9 +139,6 @@ void free_scene(rbr_ctx* ctx);
 // kernels (trace.cu)
 cudaError_t launch_trace_counts(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit,
                                 unsigned long long* totals, int* err, cudaStream_t stream);
-cudaError_t launch_trace_coop(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit, void* out, int* err,
-                              uint32_t* cursor, int grid, cudaStream_t stream);
-int trace_coop_blocks_per_sm(int any_hit);
 rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, int64_t* chosen_us);
 constexpr int kCursorRing = 64;
 // Launches a ray query with the context's chosen kernel (closest hit into rbr_hit[n] or any

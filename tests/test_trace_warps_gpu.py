@@ -68,3 +68,13 @@ def test_nodes_of_many_records(ctx, restatement):
     rays = abi.make_rays(o, (d / np.linalg.norm(d, axis=1, keepdims=True)).astype(np.float32))
     for kernel in (0, 1, 2):
         check(ctx, restatement, w, rays, kernel)
+
+
+@pytest.mark.parametrize("n", [1, 3, 4, 5, 17, 148 * 112, 148 * 112 + 1])
+def test_small_batches_by_groups(ctx, restatement, n):
+    """Kernel 0 on both sides of the rule that hands small batches over larger trees to groups of 8
+    lanes, and around a group's and a warp's share."""
+    w = scenes.random_world(400, 1500, False, seed=5)
+    ctx.upload(w)
+    assert ctx.stats().num_wide_nodes > 64
+    check(ctx, restatement, w, scenes.random_test_rays(2 * n + 16, seed=n)[:n], 0)
