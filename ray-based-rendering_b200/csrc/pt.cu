@@ -526,9 +526,21 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
     uint32_t* nextq = (d & 1) ? P.q0 : P.q1;
     uint32_t* nextc = P.counters + kCQ0 + ((d + 1) & 1);
     if (g.block == 0 && threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(P.counters + kCShade), n);
-    // one cursor per depth: the per-class launches keep the grid-stride order
-    Claim cl(P.fetch && kCls < 0 ? P.counters + kCCursor + kLine : nullptr, n, g);
-    for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
+    // A block takes blockDim.x entries at a time: in the grid-stride order, or for a long queue by
+    // claims on the depth's cursor (one cursor: the per-class launches keep the grid-stride order).
+    // The block's warps pass the phases of a vertex (lobes, each light, the BSDF sample) together:
+    // the code of a vertex is larger than the instruction cache, and warps spread over all of it
+    // waited for instruction fetches 9 of 18 cycles per issued instruction (GGX scene, depth 0).
+    // With a barrier between the phases, at 128 / 256 / 512 / 1,024 threads a block, the GGX render
+    // went from 105.6 ms to 98.5 / 96.7 / 96.2 / 100.8, the Cornell box from 882 us to 866 / 861 /
+    // 904 / 990, the foggy one from 1,506 to 1,491 / 1,481 / 1,467 / 1,544.
+    __shared__ uint32_t claimed;
+    const uint32_t stride = g.blocks * blockDim.x;
+    const bool claims = kCls < 0 && P.fetch && n / stride >= kClaimRounds;
+    for (uint32_t base = g.block * blockDim.x; base < n;) {
+        const uint32_t j = base + threadIdx.x;
+        uint32_t next = 0;  // claimed here, used at the end: the vertex covers the atomic's latency
+        if (claims && threadIdx.x == 0) next = stride + atomicAdd(P.counters + kCCursor + kLine, blockDim.x);
         const bool valid = j < n;
         uint32_t k = 0;
         bool alive = false, nee = false, to_cache = false, to_train = false, last = true, mis = false;
@@ -614,6 +626,7 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
         }
         // next-event estimation: one shadow ray per light (estimateDirectLighting)
         for (uint32_t l = 0; l < s.num_lights; ++l) {
+            __syncthreads();
             bool emit = false;
             f3 contrib, wi;
             float stmax = 0.0f;
@@ -656,6 +669,7 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
             }
         }
         // BSDF sampling, throughput update, Russian roulette, next ray
+        __syncthreads();
         bool cont = false;
         if (valid && alive && !last) {
             const float4 u = draw4(seed, pixel, sample, d, kRngBounce);
@@ -681,19 +695,34 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
         }
         const uint32_t slot = warp_append(nextc, cont);
         if (cont) nextq[slot] = k;
+        if (claims) {
+            if (threadIdx.x == 0) claimed = next;
+            __syncthreads();
+            base = claimed;
+            __syncthreads();
+        } else {
+            __syncthreads();
+            base += stride;
+        }
     }
 }
 
-// Resident blocks per SM the register budget of a shading kernel allows: the unified kernel and
-// the lobeless and delta-only classes 8 (64 registers); the glossy class 6 (80 registers) and
-// the diffuse class 7 (72), which keeps their spills small (76 / 68 bytes instead of 232 / 156).
+// Threads of a shading block (the unified kernel; see shade_body), and resident blocks of kBlock
+// threads per SM the register budget of a shading kernel allows: the unified kernel and the
+// lobeless and delta-only classes 8 (64 registers); the glossy class 6 (80 registers) and the
+// diffuse class 7 (72), which keeps their spills small (76 / 68 bytes instead of 232 / 156).
+constexpr int kShadeBlock = 256;
+template <int kCls>
+__host__ __device__ constexpr int shade_threads() {
+    return kCls < 0 ? kShadeBlock : kBlock;
+}
 template <int kCls>
 __host__ __device__ constexpr int shade_blocks() {
     return kCls == kShadeGlossy || kCls == kShadeGlossyRefl || kCls == kShadeGlossyTrans ? 6 : kCls == kShadeDiffuse ? 7 : 8;
 }
 
 template <int kMode, bool kPacked, int kCls = -1>
-__global__ void __launch_bounds__(kBlock, shade_blocks<kCls>()) k_shade(DeviceScene s, Wave w, Paths P, uint32_t d) {
+__global__ void __launch_bounds__(shade_threads<kCls>(), shade_blocks<kCls>() * kBlock / shade_threads<kCls>()) k_shade(DeviceScene s, Wave w, Paths P, uint32_t d) {
     shade_body<kMode, kPacked, kCls>(s, w, P, d, grid_span());
 }
 
@@ -930,6 +959,9 @@ __global__ void k_release(const unsigned long long* start, uint64_t release_ns) 
 
 }  // namespace
 
+// Blocks of the unified shading kernel with as many threads as `grid` blocks of the other stages.
+static int shade_grid(int grid) { return (grid * kBlock + kShadeBlock - 1) / kShadeBlock; }
+
 rbr_status read_render_counters(rbr_ctx* ctx) {
     if (!ctx->pt.counters.ptr) return RBR_OK;
     rbr_render_stats& r = ctx->last_render;
@@ -1102,7 +1134,7 @@ rbr_status render(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_params* 
             if (volumetric) {
                 if (count) k_extend<true, false, true><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
                 else k_extend<true, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
-                k_shade<2, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
+                k_shade<2, false><<<shade_grid(grid), kShadeBlock, 0, ws>>>(ctx->scene, w, P, d);
             } else {
                 if (count) k_extend<false, false, true><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
                 else k_extend<false, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
@@ -1115,7 +1147,7 @@ rbr_status render(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_params* 
                     k_shade<0, false, kShadeNone><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
                     launches += 3;
                 } else {
-                    k_shade<0, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
+                    k_shade<0, false><<<shade_grid(grid), kShadeBlock, 0, ws>>>(ctx->scene, w, P, d);
                 }
             }
             if (count) k_shadow<true><<<grid, kBlock, 0, ws>>>(ctx->scene, P, ctx->d_error);
@@ -1288,7 +1320,7 @@ rbr_status render_cached(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_p
             for (uint32_t d = 0; d < w.max_depth; ++d) {
                 k_begin<<<1, 32, 0, ws>>>(P, d);
                 k_extend<false, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
-                k_shade<1, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
+                k_shade<1, false><<<shade_grid(grid), kShadeBlock, 0, ws>>>(ctx->scene, w, P, d);
                 k_shadow<<<grid, kBlock, 0, ws>>>(ctx->scene, P, ctx->d_error);
                 launches += 4;
             }
@@ -1390,11 +1422,11 @@ cudaError_t launch_packed_wave(rbr_ctx* eng, rbr_ctx* scn, const PackedWave& pw,
         k_begin<<<1, 32, 0, stream>>>(P, d);
         if (pw.mode == 2) {
             k_extend<true, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d, eng->d_error);
-            k_shade<2, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d);
+            k_shade<2, true><<<shade_grid(grid), kShadeBlock, 0, stream>>>(scn->scene, w, P, d);
         } else {
             k_extend<false, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d, eng->d_error);
-            if (pw.mode == 1) k_shade<1, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d);
-            else k_shade<0, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d);
+            if (pw.mode == 1) k_shade<1, true><<<shade_grid(grid), kShadeBlock, 0, stream>>>(scn->scene, w, P, d);
+            else k_shade<0, true><<<shade_grid(grid), kShadeBlock, 0, stream>>>(scn->scene, w, P, d);
         }
         k_shadow<<<grid, kBlock, 0, stream>>>(scn->scene, P, eng->d_error);
     }
@@ -1589,7 +1621,7 @@ rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_
         for (uint32_t d = 0; d < w.max_depth; ++d) {
             k_begin<<<1, 32, 0, stream>>>(P, d);
             k_extend<false, false><<<grid, kBlock, 0, stream>>>(ctx->scene, w, P, d, ctx->d_error);
-            k_shade<0, false><<<grid, kBlock, 0, stream>>>(ctx->scene, w, P, d);
+            k_shade<0, false><<<shade_grid(grid), kShadeBlock, 0, stream>>>(ctx->scene, w, P, d);
             k_shadow<<<grid, kBlock, 0, stream>>>(ctx->scene, P, ctx->d_error);
         }
         k_film<<<grid, kBlock, 0, stream>>>(w, P, film_mean, nullptr);
