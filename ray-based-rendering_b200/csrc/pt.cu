@@ -5,7 +5,6 @@
 // belong to one wave, path k of a wave is sample (k % spp) of pixel (p0 + k / spp). Per wave:
 //   raygen                         camera rays for every path (counter-RNG jitter and lens)
 //   for depth = 0 .. maxDepth-1:
-//     begin    reset the per-depth queue counters and claim cursors
 //     extend   closest hit for the active queue; misses add background; hits are appended
 //              to one of six material-class queues (match.any + one atomic per class and warp)
 //     shade    per class queue: emission, next-event estimation over ALL lights (one shadow
@@ -13,7 +12,8 @@
 //              its MIS-weighted contribution), BSDF sampling, Russian roulette after depth 3;
 //              surviving paths are appended to the next active queue
 //     shadow   any hit for the shadow queue; unoccluded contributions are added to the path
-//   (extend, shade and shadow hand out a long queue by claims: see Claim)
+//   (extend, shade and shadow hand out a long queue by claims: see Claim; the surface integrator
+//   traces the shadow rays of a depth and the extension rays of the next in one launch, k_rays)
 //   film     per pixel, the sum of its samples' radiance in sample order / spp (what
 //            Film::addSample(x, y, sum / spp) stores), plus the sum of squares on request
 // The reference's estimator is reproduced, quirks included: emission only at depth 0 or after
@@ -37,23 +37,28 @@ constexpr size_t kShadowBytesLimit = size_t(2) << 30;
 
 // Counters (uint32 words). The ones that many warps update at once (queue counts, claim cursors)
 // lie on 128-byte lines of their own: the L2 serves the atomics of one line one after another, so
-// cursors and counts that share a line wait for each other.
+// cursors and counts that share a line wait for each other. Each depth has a set of its own out of
+// four: the launch that traces depth d resets the set of depth d + 2, which nothing uses then (its
+// last user, depth d - 2, ended with the launch before the last).
 constexpr int kLine = 32;
 enum : int {
-    kCQ0 = 0,                // active queue counts, ping-pong by depth parity
-    kCClass = kLine,         // kNumClasses class-queue counts, a line each
-    kCShadow = kCClass + static_cast<int>(kNumClasses) * kLine,  // shadow queue count
-    kCCursor = kCShadow + kLine,  // 3 claim cursors of one depth (Paths::fetch): extension, shading, shadow queue
-    kCQuery = kCCursor + 3 * kLine,  // radiance cache: paths ended into the cache in this wave
-    kCTrain = kCQuery + kLine,       // radiance cache: training vertices gathered in this frame
-    kCTrainBase = kCTrain + 1,       // radiance cache: kCTrain at the start of this wave
-    kCExt = kCTrain + kLine,         // 64-bit: extension rays traced
-    kCSh = kCExt + 2,                // 64-bit: shadow rays traced
-    kCShade = kCSh + 2,              // 64-bit: hit vertices shaded
-    kCTraffic = kCShade + 2,         // 4 x 64-bit (RBR_RENDER_COUNT_TRAFFIC): extension nodes, records; shadow nodes, records
+    kSQueue = 0,                                                 // active queue count
+    kSClass = kLine,                                             // kNumClasses class-queue counts, a line each
+    kSShadow = kSClass + static_cast<int>(kNumClasses) * kLine,  // shadow queue count
+    kSCursor = kSShadow + kLine,                                 // claim cursors: extension, shading, shadow queue
+    kSLines = 1 + static_cast<int>(kNumClasses) + 1 + 3,
+    kSWords = kSLines * kLine,
+    kCQuery = 4 * kSWords,      // radiance cache: paths ended into the cache in this wave
+    kCTrain = kCQuery + kLine,  // radiance cache: training vertices gathered in this frame
+    kCTrainBase = kCTrain + 1,  // radiance cache: kCTrain at the start of this wave
+    kCExt = kCTrain + kLine,    // 64-bit: extension rays traced
+    kCSh = kCExt + 2,           // 64-bit: shadow rays traced
+    kCShade = kCSh + 2,         // 64-bit: hit vertices shaded
+    kCTraffic = kCShade + 2,    // 4 x 64-bit (RBR_RENDER_COUNT_TRAFFIC): extension nodes, records; shadow nodes, records
     kCWords = kCExt + kLine
 };
 static_assert(kCExt % 2 == 0 && kCTraffic + 8 <= kCWords, "64-bit counters");
+static_assert(kSLines <= 32 && kSCursor + 3 * kLine == kSWords, "one warp resets a set");
 
 // The blocks a stage runs on: the whole grid for the wavefront kernels, one half of it for a
 // half of the persistent wave loop. Grid-stride loops start at block `block` of `blocks`.
@@ -200,6 +205,13 @@ __device__ __forceinline__ PathKey path_key(const Wave& w, const Paths& P, uint3
     return r;
 }
 
+// The counters of depth d.
+__device__ __forceinline__ uint32_t* depth_set(const Paths& P, uint32_t d) { return P.counters + (d & 3u) * kSWords; }
+// Resets them (called by one warp).
+__device__ __forceinline__ void reset_set(const Paths& P, uint32_t d, uint32_t queued = 0) {
+    if (threadIdx.x < kSLines) depth_set(P, d)[threadIdx.x * kLine] = threadIdx.x == 0 ? queued : 0u;
+}
+
 __device__ __forceinline__ uint32_t lanemask_lt() {
     uint32_t m;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
@@ -260,9 +272,10 @@ __device__ __forceinline__ void raygen_body(const CameraDev& cam, const Wave& w,
         P.rad[k] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
         P.q0[k] = k;
     }
-    if (g.block == 0 && threadIdx.x == 0) {
-        P.counters[kCQ0] = n;
-        if (w.cache_on) {
+    if (g.block == 0 && threadIdx.x < 32) {
+        reset_set(P, 0, n);
+        reset_set(P, 1);
+        if (w.cache_on && threadIdx.x == 0) {
             P.counters[kCQuery] = 0;
             P.counters[kCTrainBase] = P.counters[kCTrain];
         }
@@ -272,18 +285,6 @@ __device__ __forceinline__ void raygen_body(const CameraDev& cam, const Wave& w,
 template <bool kPacked>
 __global__ void __launch_bounds__(kBlock) k_raygen(CameraDev cam, Wave w, Paths P) {
     raygen_body<kPacked>(cam, w, P, grid_span());
-}
-
-// Resets the counters depth `d` appends to (called by one warp).
-__device__ __forceinline__ void begin_body(const Paths& P, uint32_t d) {
-    constexpr uint32_t kCounts = kNumClasses + 1 + 3;  // classes, shadow queue, cursors: consecutive lines
-    static_assert(kCCursor + 3 * kLine == kCClass + static_cast<int>(kCounts) * kLine, "one run of lines");
-    if (threadIdx.x < kCounts) P.counters[kCClass + threadIdx.x * kLine] = 0;
-    if (threadIdx.x == kCounts) P.counters[kCQ0 + ((d + 1) & 1)] = 0;
-}
-
-__global__ void k_begin(Paths P, uint32_t d) {
-    begin_body(P, d);
 }
 
 // Closest hit for the active queue; misses add the background, hits are appended to their
@@ -296,108 +297,128 @@ __global__ void k_begin(Paths P, uint32_t d) {
 // also samples the medium and traces point-light shadow rays from scatter points, gains 5 % over
 // the natural 56-register allocation (foggy Cornell box); the surface variant is unchanged.
 // kCount (RBR_RENDER_COUNT_TRAFFIC): also counts the nodes and records the traversals fetch.
-template <bool kVol, bool kPacked, bool kCount>
-__device__ __forceinline__ void extend_body(const DeviceScene& s, const Wave& w, const Paths& P, uint32_t d, int* err, Span g) {
-    const uint32_t n = P.counters[kCQ0 + (d & 1)];
+// One entry j of the queue (`valid`: it is one); every lane of the warp calls it. kBeside: shadow rays
+// are traced in the same launch.
+template <bool kVol, bool kPacked, bool kCount, bool kBeside>
+__device__ __forceinline__ void extend_entry(const DeviceScene& s, const Wave& w, const Paths& P, uint32_t d, int* err,
+                                             uint32_t j, bool valid, uint2* traffic) {
+    uint32_t* c = depth_set(P, d);
     const uint32_t* q = (d & 1) ? P.q1 : P.q0;
     uint32_t* nextq = (d & 1) ? P.q0 : P.q1;
-    uint32_t* nextc = P.counters + kCQ0 + ((d + 1) & 1);
-    if (g.block == 0 && threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(P.counters + kCExt), n);
-    uint2 traffic = make_uint2(0u, 0u);
-    Claim cl(P.fetch ? P.counters + kCCursor : nullptr, n, g);
-    for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
-        const bool valid = j < n;
-        uint32_t k = 0, cls = kNumClasses;
-        bool scatter = false, last = true, nee = false;
-        f3 T = mk(0.0f, 0.0f, 0.0f), sp = T, rd = T;
-        float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (valid) {
-            k = q[j];
-            const float4 a = P.ray[2 * k], b = P.ray[2 * k + 1];
-            float t = 0.0f;
-            // A ray with a zero or non-finite direction or origin: no traversal, no hit.
-            const uint32_t prim = degenerate(a, b) ? 0xFFFFFFFFu
-                                                   : traverse<false, kCount>(s, ld_f3(a), ld_f3(b), __int_as_float(0x7f800000),
-                                                                             t, err, &traffic);
-            P.hit[k] = make_uint2(prim, __float_as_uint(t));
-            if (kVol && s.has_medium) {
-                const float4 T4 = P.thr[k];
-                T = ld_f3(T4);
-                const PathKey key = path_key<kPacked>(w, P, k);
-                last = d + 1 >= key.max_depth;
-                nee = key.nee;
-                u = draw4(key.seed, key.pixel, key.sample, d, kRngMedium);
-                float ts = 0.0f;
-                f3 wgt;
-                scatter = medium_sample(s, prim == 0xFFFFFFFFu ? __int_as_float(0x7f800000) : t, u.x, ts, wgt);
-                T = xmul(T, wgt);
-                P.thr[k] = make_float4(T.x, T.y, T.z, T4.w);
-                if (scatter) {
-                    rd = ld_f3(b);
-                    sp = xadd(ld_f3(a), xmuls(rd, ts));  // Ray::at
-                }
+    uint32_t* nextc = depth_set(P, d + 1) + kSQueue;
+    uint32_t k = 0, cls = kNumClasses;
+    bool scatter = false, last = true, nee = false;
+    f3 T = mk(0.0f, 0.0f, 0.0f), sp = T, rd = T;
+    float4 u = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (valid) {
+        k = q[j];
+        const float4 a = P.ray[2 * k], b = P.ray[2 * k + 1];
+        float t = 0.0f;
+        // A ray with a zero or non-finite direction or origin: no traversal, no hit.
+        const uint32_t prim = degenerate(a, b) ? 0xFFFFFFFFu
+                                               : traverse<false, kCount>(s, ld_f3(a), ld_f3(b), __int_as_float(0x7f800000),
+                                                                         t, err, traffic);
+        P.hit[k] = make_uint2(prim, __float_as_uint(t));
+        if (kVol && s.has_medium) {
+            const float4 T4 = P.thr[k];
+            T = ld_f3(T4);
+            const PathKey key = path_key<kPacked>(w, P, k);
+            last = d + 1 >= key.max_depth;
+            nee = key.nee;
+            u = draw4(key.seed, key.pixel, key.sample, d, kRngMedium);
+            float ts = 0.0f;
+            f3 wgt;
+            scatter = medium_sample(s, prim == 0xFFFFFFFFu ? __int_as_float(0x7f800000) : t, u.x, ts, wgt);
+            T = xmul(T, wgt);
+            P.thr[k] = make_float4(T.x, T.y, T.z, T4.w);
+            if (scatter) {
+                rd = ld_f3(b);
+                sp = xadd(ld_f3(a), xmuls(rd, ts));  // Ray::at
             }
-            if (!scatter) {
-                if (prim == 0xFFFFFFFFu) {
-                    if (!(kVol && s.has_medium)) T = ld_f3(P.thr[k]);
+        }
+        if (!scatter) {
+            if (prim == 0xFFFFFFFFu) {
+                if (!(kVol && s.has_medium)) T = ld_f3(P.thr[k]);
+                if (kBeside) {  // shadow rays of the path may add their light at the same time
+                    atomicAdd(&P.rad[k].x, fm(T.x, s.background[0]));
+                    atomicAdd(&P.rad[k].y, fm(T.y, s.background[1]));
+                    atomicAdd(&P.rad[k].z, fm(T.z, s.background[2]));
+                } else {
                     float4 L = P.rad[k];
                     L.x = fa(L.x, fm(T.x, s.background[0]));
                     L.y = fa(L.y, fm(T.y, s.background[1]));
                     L.z = fa(L.z, fm(T.z, s.background[2]));
                     P.rad[k] = L;
-                } else {
-                    cls = s.materials[s.prim_material[prim]].cls;
                 }
+            } else {
+                cls = s.materials[s.prim_material[prim]].cls;
             }
-        }
-        {
-            // append to the class queue: lanes of one class share an atomic (match.any), one
-            // per class present in the warp; kNumClasses marks a lane with nothing to shade
-            const uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls);
-            const int leader = __ffs(peers) - 1;
-            uint32_t first = 0;
-            if (cls < kNumClasses && static_cast<int>(threadIdx.x & 31) == leader)
-                first = atomicAdd(P.counters + kCClass + cls * kLine, __popc(peers));
-            first = __shfl_sync(0xFFFFFFFFu, first, leader);
-            if (cls < kNumClasses) P.classq[cls * P.cap + first + __popc(peers & lanemask_lt())] = k;
-        }
-        if (kVol) {
-            // next-event estimation from the scatter point: point lights only, unoccluded
-            // segment of length dist, Li * Tr(dist) * phase(wo = ray direction, wi)
-            for (uint32_t l = 0; l < s.num_lights; ++l) {
-                bool emit = false;
-                f3 contrib, sd;
-                float dist = 0.0f;
-                if (scatter && nee && s.lights[l].type == RBR_LIGHT_POINT) {
-                    const LightDev& L = s.lights[l];
-                    const f3 toL = xsub(ld3(L.position), sp);
-                    dist = xlen(toL);
-                    const f3 wi = xdivs(toL, dist);
-                    sd = xnorm(wi);  // the shadow Ray's constructor normalises
-                    const f3 Li = xdivs(xmuls(ld3(L.color), L.intensity), fm(dist, dist));
-                    const float ph = hg_eval(s.hg_g, rd, wi);
-                    contrib = xmul(T, xmuls(xmul(Li, transmittance(s, dist)), ph));
-                    emit = true;
-                }
-                const uint32_t slot = warp_append(P.counters + kCShadow, emit);
-                if (emit && slot < P.shadow_cap) {
-                    float4* e = P.shadow + 3 * static_cast<size_t>(slot);
-                    e[0] = make_float4(sp.x, sp.y, sp.z, dist);
-                    e[1] = make_float4(sd.x, sd.y, sd.z, __uint_as_float(k));
-                    e[2] = make_float4(contrib.x, contrib.y, contrib.z, 0.0f);
-                }
-            }
-            // the path continues from the scatter point in a phase-function direction
-            const bool cont = scatter && !last;
-            if (cont) {
-                const f3 nd = xnorm(hg_sample(s.hg_g, rd, u.y, u.z));
-                P.ray[2 * k] = make_float4(sp.x, sp.y, sp.z, 0.0f);
-                P.ray[2 * k + 1] = make_float4(nd.x, nd.y, nd.z, 0.0f);
-            }
-            const uint32_t slot = warp_append(nextc, cont);
-            if (cont) nextq[slot] = k;
         }
     }
+    {
+        // append to the class queue: lanes of one class share an atomic (match.any), one
+        // per class present in the warp; kNumClasses marks a lane with nothing to shade
+        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, cls);
+        const int leader = __ffs(peers) - 1;
+        uint32_t first = 0;
+        if (cls < kNumClasses && static_cast<int>(threadIdx.x & 31) == leader)
+            first = atomicAdd(c + kSClass + cls * kLine, __popc(peers));
+        first = __shfl_sync(0xFFFFFFFFu, first, leader);
+        if (cls < kNumClasses) P.classq[cls * P.cap + first + __popc(peers & lanemask_lt())] = k;
+    }
+    if (kVol) {
+        // next-event estimation from the scatter point: point lights only, unoccluded
+        // segment of length dist, Li * Tr(dist) * phase(wo = ray direction, wi)
+        for (uint32_t l = 0; l < s.num_lights; ++l) {
+            bool emit = false;
+            f3 contrib, sd;
+            float dist = 0.0f;
+            if (scatter && nee && s.lights[l].type == RBR_LIGHT_POINT) {
+                const LightDev& L = s.lights[l];
+                const f3 toL = xsub(ld3(L.position), sp);
+                dist = xlen(toL);
+                const f3 wi = xdivs(toL, dist);
+                sd = xnorm(wi);  // the shadow Ray's constructor normalises
+                const f3 Li = xdivs(xmuls(ld3(L.color), L.intensity), fm(dist, dist));
+                const float ph = hg_eval(s.hg_g, rd, wi);
+                contrib = xmul(T, xmuls(xmul(Li, transmittance(s, dist)), ph));
+                emit = true;
+            }
+            const uint32_t slot = warp_append(c + kSShadow, emit);
+            if (emit && slot < P.shadow_cap) {
+                float4* e = P.shadow + 3 * static_cast<size_t>(slot);
+                e[0] = make_float4(sp.x, sp.y, sp.z, dist);
+                e[1] = make_float4(sd.x, sd.y, sd.z, __uint_as_float(k));
+                e[2] = make_float4(contrib.x, contrib.y, contrib.z, 0.0f);
+            }
+        }
+        // the path continues from the scatter point in a phase-function direction
+        const bool cont = scatter && !last;
+        if (cont) {
+            const f3 nd = xnorm(hg_sample(s.hg_g, rd, u.y, u.z));
+            P.ray[2 * k] = make_float4(sp.x, sp.y, sp.z, 0.0f);
+            P.ray[2 * k + 1] = make_float4(nd.x, nd.y, nd.z, 0.0f);
+        }
+        const uint32_t slot = warp_append(nextc, cont);
+        if (cont) nextq[slot] = k;
+    }
+}
+
+// Counts a launch's rays and resets the counters of depth d + 2.
+__device__ __forceinline__ void extend_begin(const Paths& P, uint32_t d, uint32_t n, Span g) {
+    if (g.block != 0) return;
+    if (threadIdx.x < 32) reset_set(P, d + 2);
+    if (threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(P.counters + kCExt), n);
+}
+
+template <bool kVol, bool kPacked, bool kCount>
+__device__ __forceinline__ void extend_body(const DeviceScene& s, const Wave& w, const Paths& P, uint32_t d, int* err, Span g) {
+    const uint32_t n = depth_set(P, d)[kSQueue];
+    extend_begin(P, d, n, g);
+    uint2 traffic = make_uint2(0u, 0u);
+    Claim cl(P.fetch ? depth_set(P, d) + kSCursor : nullptr, n, g);
+    for (uint32_t j = cl.take(); cl.live; j = cl.take())
+        extend_entry<kVol, kPacked, kCount, false>(s, w, P, d, err, j, j < n, &traffic);
     if (kCount) warp_add_counts(P.counters, kCTraffic, traffic);
 }
 
@@ -518,13 +539,14 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
     constexpr bool kCache = kMode == 1, kVolSurface = kMode == 2;
     constexpr uint32_t kKinds = class_kinds<kCls>();
     constexpr bool kNoNee = kCls == kShadeSpecular || kCls == kShadeNone;
+    uint32_t* counts = depth_set(P, d);
     uint32_t cnt[kNumClasses + 1];
     cnt[0] = 0;
     if (kCls < 0)
-        for (int c = 0; c < kNumClasses; ++c) cnt[c + 1] = cnt[c] + P.counters[kCClass + c * kLine];
-    const uint32_t n = kCls < 0 ? cnt[kNumClasses] : P.counters[kCClass + (kCls < 0 ? 0 : kCls) * kLine];
+        for (int c = 0; c < kNumClasses; ++c) cnt[c + 1] = cnt[c] + counts[kSClass + c * kLine];
+    const uint32_t n = kCls < 0 ? cnt[kNumClasses] : counts[kSClass + (kCls < 0 ? 0 : kCls) * kLine];
     uint32_t* nextq = (d & 1) ? P.q0 : P.q1;
-    uint32_t* nextc = P.counters + kCQ0 + ((d + 1) & 1);
+    uint32_t* nextc = depth_set(P, d + 1) + kSQueue;
     if (g.block == 0 && threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(P.counters + kCShade), n);
     // A block takes blockDim.x entries at a time: in the grid-stride order, or for a long queue by
     // claims on the depth's cursor (one cursor: the per-class launches keep the grid-stride order).
@@ -540,7 +562,7 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
     for (uint32_t base = g.block * blockDim.x; base < n;) {
         const uint32_t j = base + threadIdx.x;
         uint32_t next = 0;  // claimed here, used at the end: the vertex covers the atomic's latency
-        if (claims && threadIdx.x == 0) next = stride + atomicAdd(P.counters + kCCursor + kLine, blockDim.x);
+        if (claims && threadIdx.x == 0) next = stride + atomicAdd(counts + kSCursor + kLine, blockDim.x);
         const bool valid = j < n;
         uint32_t k = 0;
         bool alive = false, nee = false, to_cache = false, to_train = false, last = true, mis = false;
@@ -658,7 +680,7 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
                     }
                 }
             }
-            const uint32_t slot = warp_append(P.counters + kCShadow, emit);
+            const uint32_t slot = warp_append(counts + kSShadow, emit);
             if (emit && slot < P.shadow_cap) {
                 f3 so, sd;
                 spawn(h, wi, so, sd);  // after the append: fewer values live across it
@@ -726,38 +748,71 @@ __global__ void __launch_bounds__(shade_threads<kCls>(), shade_blocks<kCls>() * 
     shade_body<kMode, kPacked, kCls>(s, w, P, d, grid_span());
 }
 
-template <bool kCount>
-__device__ __forceinline__ void shadow_body(const DeviceScene& s, const Paths& P, int* err, Span g) {
-    uint32_t n = P.counters[kCShadow];
+// Shadow rays of depth d.
+__device__ __forceinline__ uint32_t shadow_begin(const Paths& P, uint32_t d, int* err, Span g) {
+    uint32_t n = depth_set(P, d)[kSShadow];
     if (n > P.shadow_cap) {
         if (g.block == 0 && threadIdx.x == 0) atomicOr(err, kErrQueueOverflow);
         n = P.shadow_cap;
     }
     if (g.block == 0 && threadIdx.x == 0) atomicAdd(reinterpret_cast<unsigned long long*>(P.counters + kCSh), n);
-    uint2 traffic = make_uint2(0u, 0u);
-    Claim cl(P.fetch ? P.counters + kCCursor + 2 * kLine : nullptr, n, g);
-    for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
-        if (j < n) {  // lanes past the end claim again with their warp
-            const float4* e = P.shadow + 3 * static_cast<size_t>(j);
-            const float4 a = e[0], b = e[1];
-            float t;
-            if (!degenerate(a, b) && !traverse<true, kCount>(s, ld_f3(a), ld_f3(b), a.w, t, err, &traffic)) {
-                const float4 c = e[2];
-                float4* L = P.rad + __float_as_uint(b.w);
-                atomicAdd(&L->x, c.x);
-                atomicAdd(&L->y, c.y);
-                atomicAdd(&L->z, c.z);
-            }
-        }
+    return n;
+}
+
+template <bool kCount>
+__device__ __forceinline__ void shadow_entry(const DeviceScene& s, const Paths& P, int* err, uint32_t j, uint2* traffic) {
+    const float4* e = P.shadow + 3 * static_cast<size_t>(j);
+    const float4 a = e[0], b = e[1];
+    float t;
+    if (!degenerate(a, b) && !traverse<true, kCount>(s, ld_f3(a), ld_f3(b), a.w, t, err, traffic)) {
+        const float4 c = e[2];
+        float4* L = P.rad + __float_as_uint(b.w);
+        atomicAdd(&L->x, c.x);
+        atomicAdd(&L->y, c.y);
+        atomicAdd(&L->z, c.z);
     }
+}
+
+template <bool kCount>
+__device__ __forceinline__ void shadow_body(const DeviceScene& s, const Paths& P, uint32_t d, int* err, Span g) {
+    const uint32_t n = shadow_begin(P, d, err, g);
+    uint2 traffic = make_uint2(0u, 0u);
+    Claim cl(P.fetch ? depth_set(P, d) + kSCursor + 2 * kLine : nullptr, n, g);
+    for (uint32_t j = cl.take(); cl.live; j = cl.take())
+        if (j < n) shadow_entry<kCount>(s, P, err, j, &traffic);  // lanes past the end claim again with their warp
     if (kCount) warp_add_counts(P.counters, kCTraffic + 4, traffic);
 }
 
 // 8 resident blocks per SM (64 registers), the grid's blocks per SM: with more registers a
 // launch would run in two waves of blocks.
 template <bool kCount = false>
-__global__ void __launch_bounds__(kBlock, 8) k_shadow(DeviceScene s, Paths P, int* err) {
-    shadow_body<kCount>(s, P, err, grid_span());
+__global__ void __launch_bounds__(kBlock, 8) k_shadow(DeviceScene s, Paths P, uint32_t d, int* err) {
+    shadow_body<kCount>(s, P, d, err, grid_span());
+}
+
+// The extension rays of depth d (> 0) and the shadow rays of depth d - 1 in one launch: neither waits for
+// the other's longest traversals, and a depth takes two launches. Entries [0, round32(n)) are the
+// extension queue's, the shadow queue's follow, so the 32 entries of a warp are of one kind.
+template <bool kPacked, bool kCount>
+__device__ __forceinline__ void rays_body(const DeviceScene& s, const Wave& w, const Paths& P, uint32_t d, int* err, Span g) {
+    const uint32_t n = depth_set(P, d)[kSQueue], n32 = (n + 31u) & ~31u;
+    extend_begin(P, d, n, g);
+    const uint32_t ns = shadow_begin(P, d - 1, err, g);
+    uint2 te = make_uint2(0u, 0u), ts = make_uint2(0u, 0u);
+    Claim cl(P.fetch ? depth_set(P, d) + kSCursor : nullptr, n32 + ns, g);
+    for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
+        if ((j & ~31u) < n32) extend_entry<false, kPacked, kCount, true>(s, w, P, d, err, j, j < n, &te);
+        else if (j - n32 < ns) shadow_entry<kCount>(s, P, err, j - n32, &ts);
+    }
+    if (kCount) {
+        warp_add_counts(P.counters, kCTraffic, te);
+        warp_add_counts(P.counters, kCTraffic + 4, ts);
+    }
+}
+
+template <bool kPacked, bool kCount = false>
+__global__ void __launch_bounds__(kBlock, 8) k_rays(DeviceScene s, Wave w, Paths P, uint32_t d, int* err) {
+    rays_body<kPacked, kCount>(s, w, P, d, err, grid_span());
 }
 
 __global__ void __launch_bounds__(kBlock) k_film(Wave w, Paths P, float* film_mean, float* film_m2) {
@@ -886,8 +941,12 @@ __device__ __noinline__ void loop_shade(const DeviceScene& s, const Paths& P, ui
     const Wave w{};
     shade_body<kMode, true, -1>(s, w, P, d, g);
 }
-__device__ __noinline__ void loop_shadow(const DeviceScene& s, const Paths& P, int* err, Span g) {
-    shadow_body<false>(s, P, err, g);
+__device__ __noinline__ void loop_shadow(const DeviceScene& s, const Paths& P, uint32_t d, int* err, Span g) {
+    shadow_body<false>(s, P, d, err, g);
+}
+__device__ __noinline__ void loop_rays(const DeviceScene& s, const Paths& P, uint32_t d, int* err, Span g) {
+    const Wave w{};
+    rays_body<true, false>(s, w, P, d, err, g);
 }
 __device__ __noinline__ void loop_film(const Paths& P, Span g) { film_packed_body(P, g); }
 
@@ -932,17 +991,19 @@ __global__ void __launch_bounds__(kBlock, 8) k_wave_loop(const __grid_constant__
         if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
         loop_raygen(P, g);
         if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
+        const bool vol = lw.mode == 2;
         for (uint32_t d = 0; d < lw.max_depth; ++d) {
-            if (g.block == 0 && threadIdx.x < 32) begin_body(P, d);
+            if (vol) loop_extend<true>(s, P, d, p.err, g);
+            else if (d == 0) loop_extend<false>(s, P, d, p.err, g);
+            else loop_rays(s, P, d, p.err, g);
             if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
-            if (lw.mode == 2) loop_extend<true>(s, P, d, p.err, g);
-            else loop_extend<false>(s, P, d, p.err, g);
-            if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
-            if (lw.mode == 2) loop_shade<2>(s, P, d, g);
+            if (vol) loop_shade<2>(s, P, d, g);
             else loop_shade<0>(s, P, d, g);
             if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
-            loop_shadow(s, P, p.err, g);
-            if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
+            if (vol || d + 1 == lw.max_depth) {
+                loop_shadow(s, P, d, p.err, g);
+                if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
+            }
         }
         loop_film(P, g);
         if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
@@ -961,6 +1022,41 @@ __global__ void k_release(const unsigned long long* start, uint64_t release_ns) 
 
 // Blocks of the unified shading kernel with as many threads as `grid` blocks of the other stages.
 static int shade_grid(int grid) { return (grid * kBlock + kShadeBlock - 1) / kShadeBlock; }
+
+// The depth loop of one wave (mode 0 path tracer, 1 with the radiance cache, 2 volumetric; split: one
+// shading launch per material class). The volumetric extension appends shadow rays of its own
+// (light samples from scatter points), so its shadow rays keep a launch per depth. Returns the launches.
+template <bool kPacked, bool kCount = false>
+static uint32_t launch_depths(const DeviceScene& s, const Wave& w, const Paths& P, uint32_t depth, int mode, bool split,
+                              int* err, int grid, cudaStream_t stream) {
+    uint32_t launches = 0;
+    for (uint32_t d = 0; d < depth; ++d) {
+        if (mode == 2) k_extend<true, kPacked, kCount><<<grid, kBlock, 0, stream>>>(s, w, P, d, err);
+        else if (d == 0) k_extend<false, kPacked, kCount><<<grid, kBlock, 0, stream>>>(s, w, P, d, err);
+        else k_rays<kPacked, kCount><<<grid, kBlock, 0, stream>>>(s, w, P, d, err);
+        if (mode == 2) {
+            k_shade<2, kPacked><<<shade_grid(grid), kShadeBlock, 0, stream>>>(s, w, P, d);
+        } else if (mode == 1) {
+            k_shade<1, kPacked><<<shade_grid(grid), kShadeBlock, 0, stream>>>(s, w, P, d);
+        } else if (split && !kPacked) {
+            k_shade<0, false, kShadeGlossy><<<grid, kBlock, 0, stream>>>(s, w, P, d);
+            k_shade<0, false, kShadeGlossyRefl><<<grid, kBlock, 0, stream>>>(s, w, P, d);
+            k_shade<0, false, kShadeGlossyTrans><<<grid, kBlock, 0, stream>>>(s, w, P, d);
+            k_shade<0, false, kShadeDiffuse><<<grid, kBlock, 0, stream>>>(s, w, P, d);
+            k_shade<0, false, kShadeSpecular><<<grid, kBlock, 0, stream>>>(s, w, P, d);
+            k_shade<0, false, kShadeNone><<<grid, kBlock, 0, stream>>>(s, w, P, d);
+            launches += kNumClasses - 1;
+        } else {
+            k_shade<0, kPacked><<<shade_grid(grid), kShadeBlock, 0, stream>>>(s, w, P, d);
+        }
+        launches += 2;
+        if (mode == 2 || d + 1 == depth) {
+            k_shadow<kCount><<<grid, kBlock, 0, stream>>>(s, P, d, err);
+            ++launches;
+        }
+    }
+    return launches;
+}
 
 rbr_status read_render_counters(rbr_ctx* ctx) {
     if (!ctx->pt.counters.ptr) return RBR_OK;
@@ -1129,31 +1225,10 @@ rbr_status render(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_params* 
         w.seed = p->seed;
         k_raygen<false><<<grid, kBlock, 0, ws>>>(cd, w, P);
         ++launches;
-        for (uint32_t d = 0; d < w.max_depth; ++d) {
-            k_begin<<<1, 32, 0, ws>>>(P, d);
-            if (volumetric) {
-                if (count) k_extend<true, false, true><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
-                else k_extend<true, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
-                k_shade<2, false><<<shade_grid(grid), kShadeBlock, 0, ws>>>(ctx->scene, w, P, d);
-            } else {
-                if (count) k_extend<false, false, true><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
-                else k_extend<false, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
-                if (ctx->pt_shade_split) {
-                    k_shade<0, false, kShadeGlossy><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
-                    k_shade<0, false, kShadeGlossyRefl><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
-                    k_shade<0, false, kShadeGlossyTrans><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
-                    k_shade<0, false, kShadeDiffuse><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
-                    k_shade<0, false, kShadeSpecular><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
-                    k_shade<0, false, kShadeNone><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d);
-                    launches += 3;
-                } else {
-                    k_shade<0, false><<<shade_grid(grid), kShadeBlock, 0, ws>>>(ctx->scene, w, P, d);
-                }
-            }
-            if (count) k_shadow<true><<<grid, kBlock, 0, ws>>>(ctx->scene, P, ctx->d_error);
-            else k_shadow<<<grid, kBlock, 0, ws>>>(ctx->scene, P, ctx->d_error);
-            launches += 4;
-        }
+        const int mode = volumetric ? 2 : 0;
+        const bool split = ctx->pt_shade_split != 0;
+        launches += count ? launch_depths<false, true>(ctx->scene, w, P, w.max_depth, mode, split, ctx->d_error, grid, ws)
+                          : launch_depths<false>(ctx->scene, w, P, w.max_depth, mode, split, ctx->d_error, grid, ws);
         k_film<<<grid, kBlock, 0, ws>>>(w, P, film_mean, film_m2);  // the wave's own pixels
         ++launches;
         ++waves;
@@ -1317,13 +1392,7 @@ rbr_status render_cached(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_p
             w.film_weight = weight;
             k_raygen<false><<<grid, kBlock, 0, ws>>>(cd, w, P);
             ++launches;
-            for (uint32_t d = 0; d < w.max_depth; ++d) {
-                k_begin<<<1, 32, 0, ws>>>(P, d);
-                k_extend<false, false><<<grid, kBlock, 0, ws>>>(ctx->scene, w, P, d, ctx->d_error);
-                k_shade<1, false><<<shade_grid(grid), kShadeBlock, 0, ws>>>(ctx->scene, w, P, d);
-                k_shadow<<<grid, kBlock, 0, ws>>>(ctx->scene, P, ctx->d_error);
-                launches += 4;
-            }
+            launches += launch_depths<false>(ctx->scene, w, P, w.max_depth, 1, false, ctx->d_error, grid, ws);
             e = cache_launch_infer(ctx, P.q_rec, w.npaths, P.counters + kCQuery, nullptr, P.rad, P.q_info, ws, P.q_sort);
             ++launches;
             if (e == cudaSuccess && train) {
@@ -1418,18 +1487,7 @@ cudaError_t launch_packed_wave(rbr_ctx* eng, rbr_ctx* scn, const PackedWave& pw,
     cudaError_t e = cudaMemsetAsync(P.counters, 0, kCWords * 4, stream);
     if (e != cudaSuccess) return e;
     k_raygen<true><<<grid, kBlock, 0, stream>>>(unused, w, P);
-    for (uint32_t d = 0; d < pw.max_depth; ++d) {
-        k_begin<<<1, 32, 0, stream>>>(P, d);
-        if (pw.mode == 2) {
-            k_extend<true, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d, eng->d_error);
-            k_shade<2, true><<<shade_grid(grid), kShadeBlock, 0, stream>>>(scn->scene, w, P, d);
-        } else {
-            k_extend<false, true><<<grid, kBlock, 0, stream>>>(scn->scene, w, P, d, eng->d_error);
-            if (pw.mode == 1) k_shade<1, true><<<shade_grid(grid), kShadeBlock, 0, stream>>>(scn->scene, w, P, d);
-            else k_shade<0, true><<<shade_grid(grid), kShadeBlock, 0, stream>>>(scn->scene, w, P, d);
-        }
-        k_shadow<<<grid, kBlock, 0, stream>>>(scn->scene, P, eng->d_error);
-    }
+    launch_depths<true>(scn->scene, w, P, pw.max_depth, pw.mode, false, eng->d_error, grid, stream);
     if (pw.mode == 1) {
         e = cache_launch_infer(scn, P.q_rec, pw.capacity, P.counters + kCQuery, nullptr, P.rad, P.q_info, stream, P.q_sort);
         if (e == cudaSuccess && pw.train)
@@ -1501,7 +1559,8 @@ cudaError_t launch_release(const unsigned long long* start, uint64_t release_ns,
 }
 
 uint32_t packed_wave_launches(const PackedWave& pw) {
-    uint32_t n = 2 + 4 * pw.max_depth;  // raygen, film, depth loop
+    // raygen, film, depth loop (launch_depths)
+    uint32_t n = 2 + (pw.mode == 2 ? 3 * pw.max_depth : 2 * pw.max_depth + (pw.max_depth ? 1 : 0));
     if (pw.mode == 1) n += 1 + (pw.train ? 1 + 4 * pw.train_steps : 0);
     return n;
 }
@@ -1514,16 +1573,19 @@ namespace {
 
 // Every GPU that loads this library holds this array until the process exits.
 __device__ __align__(256) unsigned char g_render_scratch[RBR_NOALLOC_SCRATCH_BYTES];
+__device__ __align__(256) uint32_t g_render_counters[kCWords];
 
-// Device address of g_render_scratch on the current device, looked up on every call: the
+// Device addresses of the arrays on the current device, looked up on every call: the
 // lookup allocates nothing, and a cached address would go stale if the application reset the
 // device or its primary context between calls. In host code the array's name only stands in
 // for the symbol; kernels must be given this address, never the host-side name.
-cudaError_t scratch_address(unsigned char** out) {
-    void* p = nullptr;
-    const cudaError_t e = cudaGetSymbolAddress(&p, g_render_scratch);
+cudaError_t scratch_address(unsigned char** out, uint32_t** counters) {
+    void *p = nullptr, *c = nullptr;
+    cudaError_t e = cudaGetSymbolAddress(&p, g_render_scratch);
+    if (e == cudaSuccess) e = cudaGetSymbolAddress(&c, g_render_counters);
     if (e != cudaSuccess) return e;
     *out = static_cast<unsigned char*>(p);
+    *counters = static_cast<uint32_t*>(c);
     return cudaSuccess;
 }
 
@@ -1549,7 +1611,7 @@ rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_
     // per light and path
     const uint32_t nl = std::max(1u, ctx->scene.num_lights);
     const size_t per_path = 88 + 4 * size_t(kNumClasses) + 48 * size_t(nl);
-    const size_t fixed = align256(kCWords * 4) + 8 * 256;  // counters + alignment of the eight arrays
+    const size_t fixed = 9 * 256;  // alignment of the arrays
     uint64_t cap = (RBR_NOALLOC_SCRATCH_BYTES - fixed) / per_path;
     cap = std::min<uint64_t>(cap, npix * spp);
     cap = cap / spp * spp;
@@ -1560,7 +1622,8 @@ rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_
                         "-byte scratch array (at most " +
                         std::to_string((RBR_NOALLOC_SCRATCH_BYTES - fixed) / per_path) + " samples per pixel)");
     unsigned char* base = nullptr;
-    cudaError_t e = scratch_address(&base);
+    uint32_t* counters = nullptr;
+    cudaError_t e = scratch_address(&base, &counters);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "looking up the render scratch array");
 
     size_t off = 0;
@@ -1570,7 +1633,7 @@ rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_
         return q;
     };
     Paths P;
-    P.counters = reinterpret_cast<uint32_t*>(take(kCWords * 4));
+    P.counters = counters;
     P.ray = reinterpret_cast<float4*>(take(cap * 32));
     P.thr = reinterpret_cast<float4*>(take(cap * 16));
     P.rad = reinterpret_cast<float4*>(take(cap * 16));
@@ -1618,12 +1681,7 @@ rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_
         w.use_mis = p->use_mis != 0;
         w.seed = p->seed;
         k_raygen<false><<<grid, kBlock, 0, stream>>>(cd, w, P);
-        for (uint32_t d = 0; d < w.max_depth; ++d) {
-            k_begin<<<1, 32, 0, stream>>>(P, d);
-            k_extend<false, false><<<grid, kBlock, 0, stream>>>(ctx->scene, w, P, d, ctx->d_error);
-            k_shade<0, false><<<shade_grid(grid), kShadeBlock, 0, stream>>>(ctx->scene, w, P, d);
-            k_shadow<<<grid, kBlock, 0, stream>>>(ctx->scene, P, ctx->d_error);
-        }
+        launch_depths<false>(ctx->scene, w, P, w.max_depth, 0, false, ctx->d_error, grid, stream);
         k_film<<<grid, kBlock, 0, stream>>>(w, P, film_mean, nullptr);
         e = cudaGetLastError();
     }
