@@ -464,7 +464,7 @@ __device__ __forceinline__ Hit surface(const DeviceScene& s, uint32_t prim, floa
         } else if (type == kPrimSphere) {
             outward = xdivs(xsub(h.point, mk(a.x, a.y, a.z)), a.w);  // (hitPoint - center) / radius
         } else {
-            outward = xnorm(xcross(mk(a.w, b.x, b.y), mk(b.z, b.w, c.x)));  // quad normal
+            outward = ld_f3(s.quads[__float_as_uint(c.z)]);
         }
     }
     h.front = xdot(d, outward) < 0.0f;

@@ -39,7 +39,7 @@
 //   triangle  v0.xyz, e1.xyz, e2.xyz, tag      (e1 = v1 - v0, e2 = v2 - v0, rounded as
 //                                               Triangle::intersect computes them)
 //   sphere    centre.xyz, radius, r*r, -, -, -, -, -, tag
-//   quad      origin.xyz, u.xyz, v.xyz, tag, dot(u,u), dot(v,v)
+//   quad      origin.xyz, u.xyz, v.xyz, tag, index of its normal and dot(u,u), dot(v,v)
 //   tag = primitive id | (type << 30)
 // Planes (unbounded) live outside the tree: float4 (unit normal, d) + id.
 #pragma once

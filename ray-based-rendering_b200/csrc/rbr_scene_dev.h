@@ -43,6 +43,7 @@ struct LightDev {
 struct DeviceScene {
     const uint4* nodes;      // kDevNodeWords/4 uint4 per node
     const float4* records;   // 3 float4 per leaf record
+    const float4* quads;     // per quad: unit normal, |u|^2 (index in the quad's record)
     const float4* planes;    // per plane: (unit normal, d)
     const uint32_t* plane_tags;
     uint32_t num_nodes;

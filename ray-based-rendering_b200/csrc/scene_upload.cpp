@@ -370,6 +370,18 @@ rbr_status upload_scene(rbr_ctx* ctx, const rbr_scene_desc* d) {
         std::memcpy(&records[r * kRecordWords], &words[size_t(b) * kRecordWords], kRecordWords * 4);
         prim_record[bounded_id[b]] = static_cast<uint32_t>(r);
     }
+    // quads: the unit normal as Quad's constructor computes it (Vec3::cross and normalized, rounded
+    // operation by operation) and |u|^2, whose place in the record takes their index
+    std::vector<float4> quads;
+    for (size_t r = 0; r < bvh.leaf_order.size(); ++r) {
+        uint32_t* w = &records[r * kRecordWords];
+        if (w[9] >> kTypeShift != kPrimQuad) continue;
+        float f[12];
+        std::memcpy(f, w, sizeof(f));
+        const V3 n = normalized(cross(V3{f[3], f[4], f[5]}, V3{f[6], f[7], f[8]}));
+        w[10] = static_cast<uint32_t>(quads.size());
+        quads.push_back(make_float4(n.x, n.y, n.z, f[10]));
+    }
     std::vector<float4> tri_normals;
     if (d->triangle_normals && d->num_triangles) {
         tri_normals.assign(bvh.leaf_order.size() * 3, make_float4(0, 0, 0, 0));
@@ -414,6 +426,8 @@ rbr_status upload_scene(rbr_ctx* ctx, const rbr_scene_desc* d) {
             s.tree_reach = static_cast<float>(reach * 1.001);
         }
     }
+    if ((st = upload(ctx, quads, "quad normals", &p)) != RBR_OK) return free_scene(ctx), st;
+    s.quads = static_cast<const float4*>(p);
     if ((st = upload(ctx, planes, "planes", &p)) != RBR_OK) return free_scene(ctx), st;
     s.planes = static_cast<const float4*>(p);
     if ((st = upload(ctx, plane_tags, "plane tags", &p)) != RBR_OK) return free_scene(ctx), st;
