@@ -574,6 +574,7 @@ __device__ __forceinline__ void shade_body(const DeviceScene& s, const Wave& w, 
         bs.n = 0;
         Mix mx;
         mx.total = 0.0f;
+        mx.lo = 0.0f;
         uint32_t pixel = 0, sample = 0;
         if (valid) {
             if (kCls < 0) {
