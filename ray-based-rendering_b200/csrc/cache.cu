@@ -702,10 +702,19 @@ __global__ void __launch_bounds__(128 * G, 8 / G)
 
 constexpr uint32_t smem_infer_groups(int G) { return kWBytes + G * kActBytesInfer + 8 * G + 8; }
 
+// Bias corrections 1 - beta^t of the optimiser step t that follows a batch of nsamp samples; 0 (no
+// step: the update does nothing) for an empty batch.
+__device__ __forceinline__ void adam_bias(const AdamDev& a, uint32_t nsamp, float* scalars) {
+    const double t = reinterpret_cast<const uint32_t*>(scalars)[kRcStep] + 1.0;
+    scalars[kRcBias] = nsamp ? static_cast<float>(1.0 - pow(static_cast<double>(a.beta1), t)) : 0.0f;
+    scalars[kRcBias + 1] = static_cast<float>(1.0 - pow(static_cast<double>(a.beta2), t));
+}
+
 // --------------------------------------------------------------------------------------------
-// Training: forward + loss gradient + backward + weight and grid gradients for one batch.
+// Training: forward + loss gradient + backward + weight and grid gradients for one batch. The grid
+// has one block more than the blocks that share the tiles.
 // --------------------------------------------------------------------------------------------
-__global__ void __launch_bounds__(128, 1) k_rc_train(CacheDev c, TrainBatchDev b, float* scalars, int* err) {
+__global__ void __launch_bounds__(128, 1) k_rc_train(CacheDev c, TrainBatchDev b, AdamDev a, float* scalars, int* err) {
     extern __shared__ __align__(1024) uint8_t smem[];
     uint8_t* ws = smem;
     uint8_t* act = smem + kWBytes;
@@ -716,6 +725,11 @@ __global__ void __launch_bounds__(128, 1) k_rc_train(CacheDev c, TrainBatchDev b
     const uint32_t avail = batch_avail(b, n0);
     const uint32_t nsamp = min(b.batch, avail);
     const uint32_t tiles = (nsamp + kRcTile - 1) / kRcTile;
+    const uint32_t workers = gridDim.x - 1;
+    if (blockIdx.x == workers) {  // the last block prepares the optimiser step beside the others
+        if (threadIdx.x == 0) adam_bias(a, nsamp, scalars);
+        return;
+    }
     if (blockIdx.x >= tiles) return;
     const float scale = fd(1.0f, fm(3.0f, static_cast<float>(nsamp)));
     const uint32_t tid = threadIdx.x, warp = tid >> 5;
@@ -738,7 +752,7 @@ __global__ void __launch_bounds__(128, 1) k_rc_train(CacheDev c, TrainBatchDev b
     const uint32_t act_s = tc::smem_addr(act), del_s = tc::smem_addr(del), w_s = tc::smem_addr(ws);
     uint32_t phase = 0;
     bool ok = true, first = true;
-    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += gridDim.x) {
+    for (uint32_t tile = blockIdx.x; tile < tiles && ok; tile += workers) {
         const uint32_t j = tile * kRcTile + tid;
         const bool valid = j < nsamp;
         uint32_t ridx = 0;
@@ -890,23 +904,6 @@ __global__ void __launch_bounds__(128, 1) k_rc_train(CacheDev c, TrainBatchDev b
 // --------------------------------------------------------------------------------------------
 // Adam
 // --------------------------------------------------------------------------------------------
-// Starts an optimiser step if the batch had samples: t += 1, bias corrections 1 - beta^t.
-__global__ void k_rc_adam_prep(AdamDev a, TrainBatchDev b, float* scalars) {
-    uint32_t n0 = 0;
-    const uint32_t avail = batch_avail(b, n0);
-    uint32_t* step = reinterpret_cast<uint32_t*>(scalars + kRcStep);
-    if (avail == 0 || b.batch == 0) {
-        scalars[kRcBias] = 0.0f;  // no step: the update kernels do nothing
-        return;
-    }
-    const uint32_t t = *step + 1;
-    *step = t;
-    scalars[kRcBias] = static_cast<float>(1.0 - pow(static_cast<double>(a.beta1), static_cast<double>(t)));
-    scalars[kRcBias + 1] = static_cast<float>(1.0 - pow(static_cast<double>(a.beta2), static_cast<double>(t)));
-    scalars[kRcLastLoss] = scalars[kRcLoss];
-    scalars[kRcLoss] = 0.0f;
-}
-
 __device__ __forceinline__ float adam_update(float p, float& m, float& v, float g, const AdamDev& a, float c1, float c2) {
     m = fa(fm(a.beta1, m), fm(fs(1.0f, a.beta1), g));
     v = fa(fm(a.beta2, v), fm(fm(fs(1.0f, a.beta2), g), g));
@@ -914,66 +911,82 @@ __device__ __forceinline__ float adam_update(float p, float& m, float& v, float 
     return fs(p, fd(fm(a.lr, mh), fa(__fsqrt_rn(vh), a.eps)));
 }
 
-// Dense Adam over the MLP weights (FP32 master, BF16 working copy); clears the gradients.
-__global__ void k_rc_adam_mlp(AdamDev a, float* master, float* m, float* v, float* grad, __nv_bfloat16* w,
-                              const float* scalars) {
+// One Adam step over the MLP weights (dense: FP32 master, BF16 working copy) and the hash-grid entries
+// that received a gradient (entries with a zero gradient keep their parameters and moments); clears the
+// gradients it consumed, and the last block to finish counts the step.
+// The grid's scan reads the dense gradient array, four entries a thread and pass; a touched entry's
+// master copy and moments are one 32-byte sector (interleaved state). Bound by the latency of those
+// loads: the states of a thread's touched entries are loaded together, and the next pass's gradients
+// with them (one after another, with launches of their own for the step count and the weights, 46 + 4 +
+// 6 us a step; 36 now, 38 and 42 at 8 and 16 blocks per SM).
+constexpr int kAdamBlocks = 4;  // per SM: the resident ones
+__global__ void __launch_bounds__(256) k_rc_adam(AdamDev a, float* master, float* m, float* v, float* wgrad,
+                                                 __nv_bfloat16* w, float4* state, float2* grad, __half2* h,
+                                                 uint32_t count, float* scalars) {
     const float c1 = scalars[kRcBias], c2 = scalars[kRcBias + 1];
-    if (c1 == 0.0f) return;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < kRcWeights; i += gridDim.x * blockDim.x) {
-        const float g = grad[i];
-        grad[i] = 0.0f;
-        float mi = m[i], vi = v[i];
-        const float p = adam_update(master[i], mi, vi, g, a, c1, c2);
-        m[i] = mi;
-        v[i] = vi;
-        master[i] = p;
-        w[i] = __float2bfloat16_rn(p);
-    }
-}
-
-// Adam over the hash-grid entries that received a gradient (entries with a zero gradient keep
-// their parameters and moments); clears the gradients it consumed. The scan reads the dense
-// gradient array; a touched entry's master copy and moments are one 32-byte sector
-// (interleaved state), so an update reads and writes one sector of state plus its FP16 copy.
-__device__ __forceinline__ void adam_entry(const AdamDev& a, float4* state, __half2* h, uint32_t i, float2 g,
-                                           float c1, float c2) {
-    float4* st = state + 2 * static_cast<size_t>(i);
-    float4 pm = st[0];  // master.xy, m.xy
-    const float4 vv = st[1];
-    float vx = vv.x, vy = vv.y;
-    pm.x = adam_update(pm.x, pm.z, vx, g.x, a, c1, c2);
-    pm.y = adam_update(pm.y, pm.w, vy, g.y, a, c1, c2);
-    st[0] = pm;
-    st[1] = make_float4(vx, vy, 0.0f, 0.0f);
-    h[i] = __floats2half2_rn(pm.x, pm.y);
-}
-
-__global__ void k_rc_adam_grid(AdamDev a, float4* state, float2* grad, __half2* h, uint32_t count, const float* scalars) {
-    const float c1 = scalars[kRcBias], c2 = scalars[kRcBias + 1];
-    if (c1 == 0.0f) return;
-    // Four entries per thread and pass, their gradients loaded together (two 16-byte loads), so
-    // that the scan of the (mostly untouched) gradient array keeps several loads in flight.
-    const uint32_t quads = count / 4;
-    const float4* g4 = reinterpret_cast<const float4*>(grad);
-    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < quads; q += gridDim.x * blockDim.x) {
-        const float4 ga = g4[2 * q], gb = g4[2 * q + 1];
-        const float2 gs[4] = {make_float2(ga.x, ga.y), make_float2(ga.z, ga.w), make_float2(gb.x, gb.y),
-                              make_float2(gb.z, gb.w)};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const float2 g = gs[e];
-            if (g.x == 0.0f && g.y == 0.0f) continue;
-            const uint32_t i = 4 * q + e;
-            grad[i] = make_float2(0.0f, 0.0f);
-            adam_entry(a, state, h, i, g, c1, c2);
+    const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+    if (c1 != 0.0f) {
+        const uint32_t quads = count / 4;
+        const float4* g4 = reinterpret_cast<const float4*>(grad);
+        const float4 zero = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        uint32_t q = first;
+        float4 ga = q < quads ? g4[2 * q] : zero, gb = q < quads ? g4[2 * q + 1] : zero;
+        for (uint32_t i = first; i < static_cast<uint32_t>(kRcWeights); i += stride) {
+            const float g = wgrad[i];
+            wgrad[i] = 0.0f;
+            float mi = m[i], vi = v[i];
+            const float p = adam_update(master[i], mi, vi, g, a, c1, c2);
+            m[i] = mi;
+            v[i] = vi;
+            master[i] = p;
+            w[i] = __float2bfloat16_rn(p);
         }
+        while (q < quads) {
+            const float2 gs[4] = {make_float2(ga.x, ga.y), make_float2(ga.z, ga.w), make_float2(gb.x, gb.y),
+                                  make_float2(gb.z, gb.w)};
+            bool on[4];
+            float4 pm[4], vv[4];  // master.xy and m.xy; v.xy
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                on[e] = !(gs[e].x == 0.0f && gs[e].y == 0.0f);
+                if (on[e]) {
+                    const float4* st = state + 2 * (4 * static_cast<size_t>(q) + e);
+                    pm[e] = st[0];
+                    vv[e] = st[1];
+                }
+            }
+            const uint32_t next = q + stride;
+            const bool more = next >= stride && next < quads;
+            if (more) {
+                ga = g4[2 * next];
+                gb = g4[2 * next + 1];
+            }
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                if (!on[e]) continue;
+                const uint32_t i = 4 * q + e;
+                float4* st = state + 2 * static_cast<size_t>(i);
+                grad[i] = make_float2(0.0f, 0.0f);
+                pm[e].x = adam_update(pm[e].x, pm[e].z, vv[e].x, gs[e].x, a, c1, c2);
+                pm[e].y = adam_update(pm[e].y, pm[e].w, vv[e].y, gs[e].y, a, c1, c2);
+                st[0] = pm[e];
+                st[1] = make_float4(vv[e].x, vv[e].y, 0.0f, 0.0f);
+                h[i] = __floats2half2_rn(pm[e].x, pm[e].y);
+            }
+            if (!more) break;
+            q = next;
+        }
+        // (count is a power of two of at least 2^14 entries: no entries past the last group of four)
     }
-    // entries past the last full group of four
-    for (uint32_t i = 4 * quads + blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
-        const float2 g = grad[i];
-        if (g.x == 0.0f && g.y == 0.0f) continue;
-        grad[i] = make_float2(0.0f, 0.0f);
-        adam_entry(a, state, h, i, g, c1, c2);
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        __threadfence();
+        uint32_t* word = reinterpret_cast<uint32_t*>(scalars);
+        if (atomicInc(word + kRcTicket, gridDim.x - 1) == gridDim.x - 1 && c1 != 0.0f) {
+            word[kRcStep] += 1;
+            scalars[kRcLastLoss] = scalars[kRcLoss];
+            scalars[kRcLoss] = 0.0f;
+        }
     }
 }
 
@@ -1501,17 +1514,14 @@ cudaError_t cache_launch_step(rbr_ctx* ctx, const TrainBatchDev& b, bool apply, 
     const uint32_t grid = std::max(1u, std::min<uint32_t>(tiles, ctx->num_sms));
     CacheDev dev = cs.dev;
     dev.wait_limit = ctx->cache_wait_limit;
-    k_rc_train<<<grid, 128, kSmemTrain, stream>>>(dev, b, as<float>(cs.scalars), ctx->d_error);
-    if (!apply) return cudaGetLastError();
     const AdamDev a = adam_dev(cs);
-    k_rc_adam_prep<<<1, 1, 0, stream>>>(a, b, as<float>(cs.scalars));
+    k_rc_train<<<grid + 1, 128, kSmemTrain, stream>>>(dev, b, a, as<float>(cs.scalars), ctx->d_error);
+    if (!apply) return cudaGetLastError();
     float* wm = as<float>(cs.w_master);
-    k_rc_adam_mlp<<<(kRcWeights + 255) / 256, 256, 0, stream>>>(a, wm, wm + kRcWeights, wm + 2 * kRcWeights,
-                                                                 wm + 3 * kRcWeights, as<__nv_bfloat16>(cs.w_bf16),
-                                                                 as<float>(cs.scalars));
-    k_rc_adam_grid<<<ctx->num_sms * 8, 256, 0, stream>>>(a, as<float4>(cs.grid_state), as<float2>(cs.grid_grad),
-                                                        as<__half2>(cs.grid_h), static_cast<uint32_t>(grid_entries(cs)),
-                                                        as<float>(cs.scalars));
+    k_rc_adam<<<ctx->num_sms * kAdamBlocks, 256, 0, stream>>>(a, wm, wm + kRcWeights, wm + 2 * kRcWeights, wm + 3 * kRcWeights,
+                                                    as<__nv_bfloat16>(cs.w_bf16), as<float4>(cs.grid_state),
+                                                    as<float2>(cs.grid_grad), as<__half2>(cs.grid_h),
+                                                    static_cast<uint32_t>(grid_entries(cs)), as<float>(cs.scalars));
     return cudaGetLastError();
 }
 

@@ -1416,7 +1416,7 @@ rbr_status render_cached(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_p
         }
         if (e == cudaSuccess && train) {
             e = cache_launch_train_frame(ctx, PP[0].counters + kCTrain, c1, t_half, f, stream);
-            launches += 4 * cs.cfg.train_steps;
+            launches += 2 * cs.cfg.train_steps;
         }
     }
     if (e == cudaSuccess) e = cudaEventRecord(ctx->ev_stop, stream);
@@ -1562,7 +1562,7 @@ cudaError_t launch_release(const unsigned long long* start, uint64_t release_ns,
 uint32_t packed_wave_launches(const PackedWave& pw) {
     // raygen, film, depth loop (launch_depths)
     uint32_t n = 2 + (pw.mode == 2 ? 3 * pw.max_depth : 2 * pw.max_depth + (pw.max_depth ? 1 : 0));
-    if (pw.mode == 1) n += 1 + (pw.train ? 1 + 4 * pw.train_steps : 0);
+    if (pw.mode == 1) n += 1 + (pw.train ? 1 + 2 * pw.train_steps : 0);
     return n;
 }
 
