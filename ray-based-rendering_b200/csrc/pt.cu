@@ -76,9 +76,9 @@ __device__ __forceinline__ Span grid_span() { return Span{blockIdx.x, gridDim.x}
 // drains (guided self-scheduling): a quarter of the entries left per warp, in multiples of 32
 // from 256 down to 32, so that early claims are few and the last ones leave no warp with a
 // long run of work behind the others. Atomics on the one cursor are served one after another,
-// so a short queue of cheap entries would wait on its claims (claims from four rounds up made
-// the foggy Cornell box 12 % slower): queues of fewer than kClaimRounds grid-stride rounds go
-// out in the grid-stride order.
+// so a short queue or one of cheap entries would wait on its claims: queues of fewer than
+// kClaimRounds grid-stride rounds, and those of small trees (claims_pay), go out in the
+// grid-stride order.
 // take() returns this thread's entry (entries >= n are lanes without work) and sets `live`
 // (warp-uniform) while the warp has entries: `for (j = c.take(); c.live; j = c.take())`.
 constexpr uint32_t kClaimRounds = 8;
@@ -242,6 +242,15 @@ __device__ __forceinline__ bool degenerate(float4 o, float4 d) {
 }
 
 // ------------------------------------------------------------------------------------------
+// Whether a stage that traverses rays hands out a long queue by claims: only through a tree of more than
+// kClaimNodes nodes. In a few nodes every ray costs about the same and so little that warps wait for
+// their claims (us, grid stride / claims: Cornell box at 64 spp 2,677 / 3,775, foggy 4,908 / 7,859;
+// material scene of 800 triangles and 256 spheres 5,956 / 5,540, of 2M triangles 94,753 / 89,637).
+constexpr uint32_t kClaimNodes = 64;
+__device__ __forceinline__ bool claims_pay(const DeviceScene& s, const Paths& P) {
+    return P.fetch != 0 && s.num_nodes > kClaimNodes;
+}
+
 // Starts path k of the wave: its camera ray (a, b), throughput and radiance.
 template <bool kPacked>
 __device__ __forceinline__ void start_path(const CameraDev& cam, const Wave& w, const Paths& P, uint32_t k, float4& a,
@@ -426,7 +435,7 @@ __device__ __forceinline__ void extend_body(const DeviceScene& s, const Wave& w,
     const uint32_t n = depth_set(P, d)[kSQueue];
     extend_begin(P, d, n, g);
     uint2 traffic = make_uint2(0u, 0u);
-    Claim cl(P.fetch ? depth_set(P, d) + kSCursor : nullptr, n, g);
+    Claim cl(claims_pay(s, P) ? depth_set(P, d) + kSCursor : nullptr, n, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take())
         extend_entry<kVol, kPacked, kCount, false, false>(CameraDev{}, s, w, P, d, err, j, j < n, &traffic);
     if (kCount) warp_add_counts(P.counters, kCTraffic, traffic);
@@ -442,7 +451,7 @@ __device__ __forceinline__ void first_body(const CameraDev& cam, const DeviceSce
     const uint32_t n = kPacked ? P.wave_hdr[0] : w.npaths;
     extend_begin(P, 0, n, g);
     uint2 traffic = make_uint2(0u, 0u);
-    Claim cl(P.fetch ? depth_set(P, 0) + kSCursor : nullptr, n, g);
+    Claim cl(claims_pay(s, P) ? depth_set(P, 0) + kSCursor : nullptr, n, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take())
         extend_entry<kVol, kPacked, kCount, false, true>(cam, s, w, P, 0, err, j, j < n, &traffic);
     if (kCount) warp_add_counts(P.counters, kCTraffic, traffic);
@@ -809,7 +818,7 @@ template <bool kCount>
 __device__ __forceinline__ void shadow_body(const DeviceScene& s, const Paths& P, uint32_t d, int* err, Span g) {
     const uint32_t n = shadow_begin(P, d, err, g);
     uint2 traffic = make_uint2(0u, 0u);
-    Claim cl(P.fetch ? depth_set(P, d) + kSCursor + 2 * kLine : nullptr, n, g);
+    Claim cl(claims_pay(s, P) ? depth_set(P, d) + kSCursor + 2 * kLine : nullptr, n, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take())
         if (j < n) shadow_entry<kCount>(s, P, err, j, &traffic);  // lanes past the end claim again with their warp
     if (kCount) warp_add_counts(P.counters, kCTraffic + 4, traffic);
@@ -831,7 +840,7 @@ __device__ __forceinline__ void rays_body(const DeviceScene& s, const Wave& w, c
     extend_begin(P, d, n, g);
     const uint32_t ns = shadow_begin(P, d - 1, err, g);
     uint2 te = make_uint2(0u, 0u), ts = make_uint2(0u, 0u);
-    Claim cl(P.fetch ? depth_set(P, d) + kSCursor : nullptr, n32 + ns, g);
+    Claim cl(claims_pay(s, P) ? depth_set(P, d) + kSCursor : nullptr, n32 + ns, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
         if ((j & ~31u) < n32) extend_entry<false, kPacked, kCount, true, false>(CameraDev{}, s, w, P, d, err, j, j < n, &te);
         else if (j - n32 < ns) shadow_entry<kCount>(s, P, err, j - n32, &ts);
