@@ -13,6 +13,8 @@
 
 namespace rbr {
 
+constexpr int kCursorRing = 64;
+
 // A device allocation owned by the context.
 struct DevBuf {
     void* ptr = nullptr;
@@ -52,9 +54,10 @@ struct rbr_ctx {
     rbr::DevBuf stage_in, stage_out;
     // device error word (rbr::kErr*)
     int* d_error = nullptr;
-    // work cursors of the persistent trace kernel: one per launch, taken round-robin so that
-    // launches overlapping on different streams never share one
+    // work cursors of the persistent trace kernels: one per launch, taken round-robin, and the end of
+    // the launch that used each last
     uint32_t* d_cursors = nullptr;
+    cudaEvent_t cursor_done[rbr::kCursorRing] = {};
     uint32_t cursor_next = 0;
     // tunables (rbr_param_set / rbr_autotune)
     int trace_kernel = 0;          // 0: adaptive persistent warps, 1: warp traversal with lane refill, 2: warp-cooperative
@@ -140,7 +143,6 @@ void free_scene(rbr_ctx* ctx);
 cudaError_t launch_trace_counts(const DeviceScene& s, const rbr_ray* rays, uint32_t n, int any_hit,
                                 unsigned long long* totals, int* err, cudaStream_t stream);
 rbr_status autotune_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, int64_t* chosen_us);
-constexpr int kCursorRing = 64;
 // Launches a ray query with the context's chosen kernel (closest hit into rbr_hit[n] or any
 // hit into uint8_t[n]).
 // slot 0 or 1: which sort scratch a sorted launch uses (launches in flight on two streams).
