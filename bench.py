@@ -261,14 +261,15 @@ def render_scene(which):
 
 # Algorithmic bytes of the wavefront path tracer, per event (the fixed record sizes its kernels
 # read and write; traversal bytes come from counted nodes and leaf records, 96 B and 48 B):
-#   camera path (k_raygen: ray 32 + throughput 16 + radiance 16 + queue 4; k_film: radiance 16)
-#   extension ray (k_extend: queue 4 + ray 32 + hit 8 + class queue 4)
+#   camera path (k_first: ray 32 + throughput 16 + radiance 16 written, less the queue entry and ray,
+#                36, that depth 0 does not read; k_film: radiance 16)
+#   extension ray (k_first, k_rays: queue 4 + ray 32 + hit 8 + class queue 4)
 #   shaded vertex (k_shade: class queue 4 + hit 8 + ray 32 + throughput 16 + leaf record 48 +
 #                  material index 4 + material 44)
 #   continuation (k_shade: next ray 32 + throughput 16 + queue 4)
-#   shadow ray (k_shade writes and k_shadow reads its 48 B record)
+#   shadow ray (k_shade writes and k_rays or k_shadow reads its 48 B record)
 #   pixel (k_film: 12 B of RGB film written)
-PT_BYTES = {"path": 68 + 16, "extension_ray": 48, "shaded_vertex": 156, "continuation": 52, "shadow_ray": 96,
+PT_BYTES = {"path": 64 - 36 + 16, "extension_ray": 48, "shaded_vertex": 156, "continuation": 52, "shadow_ray": 96,
             "pixel": 12, "node": 96, "leaf_record": 48}
 
 
@@ -880,7 +881,7 @@ def main():
                          "algorithmic_bytes_per_launch": alg_bytes,
                          "per_ray": {"nodes": nodes / n, "leaf_records": recs / n,
                                      "bytes": alg_bytes / n},
-                         "kernel": "k_trace_closest" if not tuned.get("trace.order") else
+                         "kernel": "k_trace (closest hit)" if not tuned.get("trace.order") else
                          "k_trace_closest_perm (timed with its ray sort: the whole call)",
                          "avg_launch_ms": avg_launch_s * 1e3},
             "cpu_baseline": base,
