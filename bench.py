@@ -231,7 +231,7 @@ def config_block():
                         "seed 0) vs a 1,310,720-triangle displaced icosphere (level 8, radius 10, 4-octave value "
                         "noise, amplitude 0.1); closest hit",
             "rays_per_step": 1 << RAYS_LOG2, "triangles": 20 * 4 ** ICO_LEVEL,
-            "l2": "inputs larger than L2: 134 MB of rays per step (the 70 MB BVH stays L2-resident by design)",
+            "l2": "inputs larger than L2: 134 MB of rays per step (the 77 MB BVH stays L2-resident by design)",
             "parallelism": "replicas (each GPU its own rays)"}
 
 

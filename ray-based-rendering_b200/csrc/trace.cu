@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
                 idx = perm ? __ldg(perm + j) : j;
                 const float4 a = ray_word<kStream>(rays + 2 * static_cast<size_t>(idx));
                 const float4 b = ray_word<kStream>(rays + 2 * static_cast<size_t>(idx) + 1);
-                // finished at once: takes another ray in this round
+                // finished at once: takes another ray in the same pass
                 if (lane_begin<kAny>(s, w, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, lr)) answer();
             }
             run = min(end, run + __popc(need));  // each round consumes at least one ray
@@ -385,7 +385,7 @@ __global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const 
                 idx = j;
                 const float4 a = __ldg(rays + 2 * static_cast<size_t>(idx));
                 const float4 b = __ldg(rays + 2 * static_cast<size_t>(idx) + 1);
-                // finished at once: takes another ray in this round
+                // finished at once: takes another ray in the same pass
                 if (group_begin<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, st, anyhit)) answer();
             }
             run = min(end, run + __popc(need));
