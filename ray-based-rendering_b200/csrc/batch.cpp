@@ -415,7 +415,7 @@ rbr_status run(rbr_batch* b, std::vector<Req>& reqs, cudaStream_t stream) {
             pw.train_thresh = static_cast<uint32_t>(std::min(4294967295.0, frac * 4294967296.0));
             pw.train_steps = scn->cache.cfg.train_steps;
         }
-        s.kernel_launches += packed_wave_launches(pw);
+        s.kernel_launches += packed_wave_launches(scn, pw);
         s.segments += static_cast<uint32_t>(w.segs.size());
         s.paths += w.paths;
         if (b->cfg.use_graphs) {

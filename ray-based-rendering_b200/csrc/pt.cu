@@ -5,8 +5,8 @@
 // belong to one wave, path k of a wave is sample (k % spp) of pixel (p0 + k / spp). Per wave:
 //   for depth = 0 .. maxDepth-1:
 //     extend   closest hit for the active queue (at depth 0 the paths are started here: camera rays
-//              with counter-RNG jitter and lens); misses add background; hits are appended
-//              to one of six material-class queues (match.any + one atomic per class and warp)
+//              with counter-RNG jitter and lens); hits are appended to one of six material-class
+//              queues (match.any + one atomic per class and warp)
 //     shade    per class queue: emission, next-event estimation over ALL lights (one shadow
 //              ray per light with a non-black BSDF value, appended to the shadow queue with
 //              its MIS-weighted contribution), BSDF sampling, Russian roulette after depth 3;
@@ -14,6 +14,7 @@
 //     shadow   any hit for the shadow queue; unoccluded contributions are added to the path
 //   (extend, shade and shadow hand out a long queue by claims: see Claim; the surface integrator
 //   traces the shadow rays of a depth and the extension rays of the next in one launch, k_rays)
+//   background  where it is lit: added to the paths whose last ray hit nothing (background_body)
 //   film     per pixel, the sum of its samples' radiance in sample order / spp (what
 //            Film::addSample(x, y, sum / spp) stores), plus the sum of squares on request
 // The reference's estimator is reproduced, quirks included: emission only at depth 0 or after
@@ -298,8 +299,36 @@ __global__ void __launch_bounds__(kBlock) k_raygen(CameraDev cam, Wave w, Paths 
     raygen_body<kPacked>(cam, w, P, grid_span());
 }
 
-// Closest hit for the active queue; misses add the background, hits are appended to their
-// material-class queue. kVol (VolumetricPathIntegrator::Li, volumetric_path_integrator.cpp:
+// The light of a ray that hits nothing. The surface integrator traces the shadow rays of a depth beside
+// the extension rays of the next, so a background that is not black is added when a wave's depths are
+// done, to the paths whose last ray hit nothing: after the path's shadow rays, the same sum in every
+// run. (Added by atomics beside them, a scene of one light repeated to an ulp only.)
+__device__ __forceinline__ void add_background(const DeviceScene& s, const Paths& P, uint32_t k, f3 T) {
+    float4 L = P.rad[k];
+    L.x = fa(L.x, fm(T.x, s.background[0]));
+    L.y = fa(L.y, fm(T.y, s.background[1]));
+    L.z = fa(L.z, fm(T.z, s.background[2]));
+    P.rad[k] = L;
+}
+__host__ __device__ __forceinline__ bool lit_background(const DeviceScene& s) {
+    return s.background[0] != 0.0f || s.background[1] != 0.0f || s.background[2] != 0.0f;
+}
+
+template <bool kPacked>
+__device__ __forceinline__ void background_body(const DeviceScene& s, const Wave& w, const Paths& P, Span g) {
+    const uint32_t n = kPacked ? P.wave_hdr[0] : w.npaths;
+    const uint32_t stride = g.blocks * blockDim.x;
+    for (uint32_t k = g.block * blockDim.x + threadIdx.x; k < n; k += stride)
+        if (P.hit[k].x == 0xFFFFFFFFu) add_background(s, P, k, ld_f3(P.thr[k]));
+}
+
+template <bool kPacked>
+__global__ void __launch_bounds__(kBlock) k_background(DeviceScene s, Wave w, Paths P) {
+    background_body<kPacked>(s, w, P, grid_span());
+}
+
+// Closest hit for the active queue; hits are appended to their material-class queue. kVol
+// (VolumetricPathIntegrator::Li, volumetric_path_integrator.cpp:
 // 11-43): a distance is sampled in the scene's medium up to the hit (or infinity) and the
 // throughput multiplied by the medium weight; a scattering event is handled here: next-event
 // estimation towards point lights (directLightingVolume, :92-118) and a phase-function sample
@@ -308,10 +337,9 @@ __global__ void __launch_bounds__(kBlock) k_raygen(CameraDev cam, Wave w, Paths 
 // also samples the medium and traces point-light shadow rays from scatter points, gains 5 % over
 // the natural 56-register allocation (foggy Cornell box); the surface variant is unchanged.
 // kCount (RBR_RENDER_COUNT_TRAFFIC): also counts the nodes and records the traversals fetch.
-// One entry j of the queue (`valid`: it is one); every lane of the warp calls it. kBeside: shadow rays
-// are traced in the same launch.
+// One entry j of the queue (`valid`: it is one); every lane of the warp calls it.
 // kFirst: entry j is path j of the wave, started here (depth 0).
-template <bool kVol, bool kPacked, bool kCount, bool kBeside, bool kFirst>
+template <bool kVol, bool kPacked, bool kCount, bool kFirst>
 __device__ __forceinline__ void extend_entry(const CameraDev& cam, const DeviceScene& s, const Wave& w, const Paths& P,
                                              uint32_t d, int* err, uint32_t j, bool valid, uint2* traffic) {
     uint32_t* c = depth_set(P, d);
@@ -357,17 +385,14 @@ __device__ __forceinline__ void extend_entry(const CameraDev& cam, const DeviceS
         }
         if (!scatter) {
             if (prim == 0xFFFFFFFFu) {
-                if (!(kVol && s.has_medium)) T = ld_f3(P.thr[k]);
-                if (kBeside) {  // shadow rays of the path may add their light at the same time
-                    atomicAdd(&P.rad[k].x, fm(T.x, s.background[0]));
-                    atomicAdd(&P.rad[k].y, fm(T.y, s.background[1]));
-                    atomicAdd(&P.rad[k].z, fm(T.z, s.background[2]));
-                } else {
-                    float4 L = P.rad[k];
-                    L.x = fa(L.x, fm(T.x, s.background[0]));
-                    L.y = fa(L.y, fm(T.y, s.background[1]));
-                    L.z = fa(L.z, fm(T.z, s.background[2]));
-                    P.rad[k] = L;
+                if (kVol) {
+                    if (!s.has_medium) T = ld_f3(P.thr[k]);
+                    add_background(s, P, k, T);
+                } else if (!lit_background(s)) {  // adds zero, but NaN to a throughput that is not finite
+                    const float4 Z = P.thr[k];
+                    if (fm(Z.x, 0.0f) != 0.0f) atomicAdd(&P.rad[k].x, fm(Z.x, 0.0f));
+                    if (fm(Z.y, 0.0f) != 0.0f) atomicAdd(&P.rad[k].y, fm(Z.y, 0.0f));
+                    if (fm(Z.z, 0.0f) != 0.0f) atomicAdd(&P.rad[k].z, fm(Z.z, 0.0f));
                 }
             } else {
                 cls = s.materials[s.prim_material[prim]].cls;
@@ -437,7 +462,7 @@ __device__ __forceinline__ void extend_body(const DeviceScene& s, const Wave& w,
     uint2 traffic = make_uint2(0u, 0u);
     Claim cl(claims_pay(s, P) ? depth_set(P, d) + kSCursor : nullptr, n, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take())
-        extend_entry<kVol, kPacked, kCount, false, false>(CameraDev{}, s, w, P, d, err, j, j < n, &traffic);
+        extend_entry<kVol, kPacked, kCount, false>(CameraDev{}, s, w, P, d, err, j, j < n, &traffic);
     if (kCount) warp_add_counts(P.counters, kCTraffic, traffic);
 }
 
@@ -453,7 +478,7 @@ __device__ __forceinline__ void first_body(const CameraDev& cam, const DeviceSce
     uint2 traffic = make_uint2(0u, 0u);
     Claim cl(claims_pay(s, P) ? depth_set(P, 0) + kSCursor : nullptr, n, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take())
-        extend_entry<kVol, kPacked, kCount, false, true>(cam, s, w, P, 0, err, j, j < n, &traffic);
+        extend_entry<kVol, kPacked, kCount, true>(cam, s, w, P, 0, err, j, j < n, &traffic);
     if (kCount) warp_add_counts(P.counters, kCTraffic, traffic);
 }
 
@@ -842,7 +867,7 @@ __device__ __forceinline__ void rays_body(const DeviceScene& s, const Wave& w, c
     uint2 te = make_uint2(0u, 0u), ts = make_uint2(0u, 0u);
     Claim cl(claims_pay(s, P) ? depth_set(P, d) + kSCursor : nullptr, n32 + ns, g);
     for (uint32_t j = cl.take(); cl.live; j = cl.take()) {
-        if ((j & ~31u) < n32) extend_entry<false, kPacked, kCount, true, false>(CameraDev{}, s, w, P, d, err, j, j < n, &te);
+        if ((j & ~31u) < n32) extend_entry<false, kPacked, kCount, false>(CameraDev{}, s, w, P, d, err, j, j < n, &te);
         else if (j - n32 < ns) shadow_entry<kCount>(s, P, err, j - n32, &ts);
     }
     if (kCount) {
@@ -999,6 +1024,10 @@ __device__ __noinline__ void loop_rays(const DeviceScene& s, const Paths& P, uin
     const Wave w{};
     rays_body<true, false>(s, w, P, d, err, g);
 }
+__device__ __noinline__ void loop_background(const DeviceScene& s, const Paths& P, Span g) {
+    const Wave w{};
+    background_body<true>(s, w, P, g);
+}
 __device__ __noinline__ void loop_film(const Paths& P, Span g) { film_packed_body(P, g); }
 
 struct LoopParams {
@@ -1062,6 +1091,10 @@ __global__ void __launch_bounds__(kBlock, 8) k_wave_loop(const __grid_constant__
                 if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
             }
         }
+        if (!vol && lw.max_depth != 0 && lit_background(s)) {
+            loop_background(s, P, g);
+            if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
+        }
         loop_film(P, g);
         if (!grid_barrier(bar, gen, per, p.limit_ns, p.err)) return;
         if (g.block == 0 && threadIdx.x == 0) p.stamps[1 + wi] = global_ns();
@@ -1116,6 +1149,10 @@ static uint32_t launch_depths(const CameraDev& cam, const DeviceScene& s, const 
             k_shadow<kCount><<<grid, kBlock, 0, stream>>>(s, P, d, err);
             ++launches;
         }
+    }
+    if (mode != 2 && depth != 0 && lit_background(s)) {
+        k_background<kPacked><<<grid, kBlock, 0, stream>>>(s, w, P);
+        ++launches;
     }
     return launches;
 }
@@ -1618,9 +1655,10 @@ cudaError_t launch_release(const unsigned long long* start, uint64_t release_ns,
     return cudaGetLastError();
 }
 
-uint32_t packed_wave_launches(const PackedWave& pw) {
+uint32_t packed_wave_launches(const rbr_ctx* scn, const PackedWave& pw) {
     // film, paths and depth loop (launch_depths)
     uint32_t n = 1 + (pw.max_depth == 0 ? 1 : pw.mode == 2 ? 3 * pw.max_depth : 2 * pw.max_depth + 1);
+    if (pw.mode != 2 && pw.max_depth != 0 && lit_background(scn->scene)) ++n;
     if (pw.mode == 1) n += 1 + (pw.train ? 1 + 2 * pw.train_steps : 0);
     return n;
 }

@@ -208,7 +208,7 @@ cudaError_t launch_wave_loop(rbr_ctx* eng, const std::vector<rbr_ctx*>& scenes, 
                              int halves, cudaStream_t stream, int* grid_out);
 cudaError_t launch_stamp(unsigned long long* at, cudaStream_t stream);
 cudaError_t launch_release(const unsigned long long* start, uint64_t release_ns, cudaStream_t stream);
-uint32_t packed_wave_launches(const PackedWave& pw);
+uint32_t packed_wave_launches(const rbr_ctx* scn, const PackedWave& pw);
 
 rbr_status render_noalloc(rbr_ctx* ctx, const rbr_camera* cam, const rbr_render_params* p, float* film_mean,
                           cudaStream_t stream);
