@@ -214,6 +214,7 @@ __device__ __forceinline__ uint32_t lane_mask_lt() {
 // With `perm` (sorted rays), position j of the order is ray perm[j]. kRefillOnly: every warp goes
 // the second way.
 constexpr int kPersistBlock = 128;
+constexpr uint32_t kPersistChunk = 4;  // first runs in a block's own chunk, at most
 constexpr uint32_t kClaimRays = 32;
 constexpr uint32_t kSmallTree = 64;      // nodes
 constexpr uint32_t kAdaptiveRefill = 6;  // idle lanes before a refill (4 to 8 measured within 2 %)
@@ -239,34 +240,64 @@ __device__ __forceinline__ bool coherent_pays(const DeviceScene& s, uint32_t n) 
     return n / 32u >= s.num_nodes && (n >= (1u << 20) || s.num_nodes <= kSmallTree);
 }
 
-// Any rays where no lane would be refilled and the traversals are short: their latency is least
-// one thread per ray (1,001 rays over 260 primitives: 15.1 us against 17.6 by warp traversal).
-__device__ __forceinline__ bool few_rays_small_tree(const DeviceScene& s, uint32_t n, uint32_t first) {
-    return n <= first && s.num_nodes <= kSmallTree;
+// Any rays where no lane would be refilled (every ray is in a first run) and the traversals are short:
+// their latency is least one thread per ray (1,001 rays over 260 primitives: 15.1 us against 17.6 by warp
+// traversal).
+__device__ __forceinline__ bool few_rays_small_tree(const DeviceScene& s, bool first_runs_only) {
+    return first_runs_only && s.num_nodes <= kSmallTree;
 }
+
+// The rays a block works on: all n of them, claimed from a cursor that the grid shares, or where there is
+// none (and kOwn) `chunk` consecutive ones, claimed from a cursor of the block's own. The warps' first
+// runs go by their index in the grid or the block.
+template <uint32_t kBlockRays, bool kOwn>
+struct BlockRays {
+    uint32_t n, chunk;
+    uint32_t *cursor, *own;
+
+    __device__ __forceinline__ uint32_t begin() const { return blockIdx.x * (kOwn && !cursor ? chunk : kBlockRays); }
+    __device__ __forceinline__ bool first_runs_only() const { return !cursor && chunk == kBlockRays; }
+    __device__ __forceinline__ void start() const {
+        if (!kOwn || cursor || chunk == kBlockRays) return;
+        if (threadIdx.x == 0) *own = 0;
+        __syncthreads();
+    }
+    // The next `count` rays for a warp (run to end); false when there are none.
+    __device__ __forceinline__ bool claim(uint32_t count, uint32_t& run, uint32_t& end) const {
+        uint32_t b = 0, limit = n, first = gridDim.x * kBlockRays;
+        if (!kOwn && !cursor) return false;
+        if (!kOwn || cursor) {
+            if ((threadIdx.x & 31u) == 0) b = atomicAdd(cursor, count);
+        } else {
+            const uint32_t from = blockIdx.x * chunk, rays = min(chunk, n - from);
+            if (rays <= kBlockRays) return false;
+            first = from + kBlockRays;
+            limit = from + rays;
+            if ((threadIdx.x & 31u) == 0) b = atomicAdd(own, count);
+        }
+        run = first + __shfl_sync(0xFFFFFFFFu, b, 0);
+        if (run < first || run >= limit) return false;  // past the end (run < first: past 2^32)
+        end = run + min(count, limit - run);
+        return true;
+    }
+};
 
 template <bool kAny, bool kStream, bool kRefillOnly>
 __global__ void __launch_bounds__(kPersistBlock, 8)
     k_trace(DeviceScene s, const float4* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ perm,
-            uint2* __restrict__ hits, uint8_t* __restrict__ occ, int* err, uint32_t* cursor, uint32_t refill_min) {
+            uint2* __restrict__ hits, uint8_t* __restrict__ occ, int* err, uint32_t* cursor, uint32_t chunk,
+            uint32_t refill_min) {
     __shared__ WarpRays shared[kPersistBlock / 32];
+    __shared__ uint32_t own;
     WarpRays& w = shared[threadIdx.x >> 5];
     const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t first = gridDim.x * kPersistBlock;  // rays before this belong to the warps' first runs
-    uint32_t run = blockIdx.x * kPersistBlock + (threadIdx.x & ~31u);  // warp-uniform
-    if (run >= n) return;
+    const BlockRays<kPersistBlock, true> mine{n, chunk, cursor, &own};
+    mine.start();
+    uint32_t run = mine.begin() + (threadIdx.x & ~31u);  // warp-uniform
+    if (run < mine.begin() || run >= n) return;
     uint32_t end = run + min(kClaimRays, n - run);  // warp-uniform
-    // the warp's next run of rays; false when there is none (no cursor: every ray is in a first run)
-    auto claim = [&]() {
-        if (!cursor) return false;
-        uint32_t b = 0;
-        if (lane == 0) b = atomicAdd(cursor, kClaimRays);
-        run = first + __shfl_sync(0xFFFFFFFFu, b, 0);
-        if (run < first || run >= n) return false;  // past the end (run < first: past 2^32)
-        end = run + min(kClaimRays, n - run);
-        return true;
-    };
-    if (!kRefillOnly && (coherent_pays(s, n) || few_rays_small_tree(s, n, first))) {
+    auto claim = [&]() { return mine.claim(kClaimRays, run, end); };
+    if (!kRefillOnly && (coherent_pays(s, n) || few_rays_small_tree(s, mine.first_runs_only()))) {
         uint32_t i = run + lane;
         bool valid = i < end;
         float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
@@ -274,7 +305,7 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
             a = ray_word<kStream>(rays + 2 * static_cast<size_t>(i));
             b = ray_word<kStream>(rays + 2 * static_cast<size_t>(i) + 1);
         }
-        if (few_rays_small_tree(s, n, first) || coherent_rays(s, valid, a, b)) {
+        if (few_rays_small_tree(s, mine.first_runs_only()) || coherent_rays(s, valid, a, b)) {
             while (true) {
                 if (valid) {
                     float t = 0.0f;
@@ -337,28 +368,24 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
 // rbr_device.cuh) and takes the next ray of the warp's chunk when its own is done.
 // ------------------------------------------------------------------------------------------
 constexpr int kCoopBlock = 128;
+constexpr uint32_t kCoopChunk = 16;
 
-template <bool kAny>
-__global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const float4* __restrict__ rays, uint32_t n,
-                                                           uint2* __restrict__ hits, uint8_t* __restrict__ occ,
-                                                           int* err, uint32_t* cursor) {
+template <bool kAny, bool kOwn>
+__device__ __forceinline__ void trace_coop_body(const DeviceScene& s, const float4* __restrict__ rays, uint32_t n,
+                                                uint2* __restrict__ hits, uint8_t* __restrict__ occ, int* err,
+                                                uint32_t* cursor, uint32_t chunk) {
+    __shared__ uint32_t own;
     const GroupLanes g = group_lanes();
     // A warp's first run is four rays, one per group, by its index; then an equal share of the rest
-    // for every warp by claims on the cursor (none where every ray is in a first run).
-    const uint32_t warps = gridDim.x * (kCoopBlock / 32), first = 4u * warps;
-    const uint32_t share = min(32u, max(4u, n / warps));
-    uint32_t run = 4u * (blockIdx.x * (kCoopBlock / 32) + (threadIdx.x >> 5));  // warp-uniform
-    if (run >= n) return;
+    // for every warp by claims (four at a time of a block's own chunk).
+    const BlockRays<kCoopBlock / 8, kOwn> mine{n, chunk, cursor, &own};
+    mine.start();
+    uint32_t run = mine.begin() + 4u * (threadIdx.x >> 5);  // warp-uniform
+    if (run < mine.begin() || run >= n) return;
     uint32_t end = run + min(4u, n - run);    // warp-uniform
     bool exhausted = false;                   // warp-uniform
     auto claim = [&]() {
-        if (!cursor) return false;
-        uint32_t b = 0;
-        if ((threadIdx.x & 31u) == 0) b = atomicAdd(cursor, share);
-        run = first + __shfl_sync(0xFFFFFFFFu, b, 0);
-        if (run < first || run >= n) return false;  // past the end (run < first: past 2^32)
-        end = run + min(share, n - run);
-        return true;
+        return mine.claim(kOwn ? 4u : min(32u, max(4u, n / (gridDim.x * (kCoopBlock / 32)))), run, end);
     };
     uint32_t idx = 0xFFFFFFFFu;               // group-uniform
     uint32_t anyhit = 0;
@@ -396,22 +423,45 @@ __global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const 
     }
 }
 
+template <bool kAny>
+__global__ void __launch_bounds__(kCoopBlock) k_trace_coop(DeviceScene s, const float4* __restrict__ rays, uint32_t n,
+                                                           uint2* __restrict__ hits, uint8_t* __restrict__ occ,
+                                                           int* err, uint32_t* cursor, uint32_t chunk) {
+    trace_coop_body<kAny, false>(s, rays, n, hits, occ, err, cursor, chunk);
+}
+
+// Blocks with chunks of their own: another kernel, since the shared cursor's has no registers to spare
+// (with both in one, 8,192 rays through 1.3M triangles 50 -> 54 us).
+template <bool kAny>
+__global__ void __launch_bounds__(kCoopBlock, 8)
+    k_trace_coop_own(DeviceScene s, const float4* __restrict__ rays, uint32_t n, uint2* __restrict__ hits,
+                     uint8_t* __restrict__ occ, int* err, uint32_t* cursor, uint32_t chunk) {
+    trace_coop_body<kAny, true>(s, rays, n, hits, occ, err, cursor, chunk);
+}
+
 }  // namespace
 
-// A cursor of zero for a launch of `grid` blocks whose first runs are `block_rays` rays a block; none
-// where these are all n rays. A cursor of the ring may still be in use by a launch on another stream
-// (64 short launches beside one long one): its event makes `stream` wait for that launch. A launch
-// captured into a graph can run beside any later one, so it gets no cursor but a grid for all rays.
+// How a launch of up to *grid resident blocks with first runs of `block_rays` rays a block hands out n
+// rays: nothing to claim where the first runs are all of them, else a cursor of zero. A cursor of the ring
+// may still be in use by a launch on another stream (64 short launches beside one long one): its event
+// makes `stream` wait for that launch. A launch captured into a graph can run beside any later one, so it
+// gets no cursor: *grid becomes blocks for all rays, each with a chunk of up to `most` first runs of its
+// own, so that lanes are refilled within a block and the hardware hands out the blocks. 2^22 uniform rays
+// through 330 K triangles, kernel 0: 1,099 us (951 by a cursor, 1,485 with first runs only, 1,082 with the
+// resident blocks taking runs in turn, which lost a quarter on camera rays: 691 -> 897); kernel 2: 3,560
+// (3,240; 4,444).
 // The events cost nothing that shows: 2^22 uniform rays 1,048 us before, 1,032 with them (another run).
-static cudaError_t take_cursor(rbr_ctx* ctx, uint32_t n, uint32_t block_rays, uint32_t* grid, uint32_t** cursor,
-                               cudaEvent_t* done, cudaStream_t stream) {
+static cudaError_t take_cursor(rbr_ctx* ctx, uint32_t n, uint32_t block_rays, uint32_t most, uint32_t* grid,
+                               uint32_t* chunk, uint32_t** cursor, cudaEvent_t* done, cudaStream_t stream) {
     *cursor = nullptr;
+    *chunk = block_rays;
     if (n <= *grid * block_rays) return cudaSuccess;
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(stream, &capture);
     if (e != cudaSuccess) return e;
     if (capture != cudaStreamCaptureStatusNone) {
-        *grid = static_cast<uint32_t>((uint64_t(n) + block_rays - 1) / block_rays);
+        *chunk *= std::min(n / (*grid * block_rays), most);
+        *grid = static_cast<uint32_t>((uint64_t(n) + *chunk - 1) / *chunk);
         return cudaSuccess;
     }
     const uint32_t slot = ctx->cursor_next++ % kCursorRing;
@@ -434,13 +484,14 @@ static cudaError_t launch_trace_coop(rbr_ctx* ctx, const rbr_ray* rays, uint32_t
     constexpr uint32_t kBlockRays = kCoopBlock / 8;
     uint32_t grid = static_cast<uint32_t>(std::max<uint64_t>(
         1, std::min<uint64_t>(uint64_t(ctx->num_sms) * per_sm, (uint64_t(n) + kBlockRays - 1) / kBlockRays)));
-    uint32_t* cursor = nullptr;
+    uint32_t *cursor = nullptr, chunk = 0;
     cudaEvent_t done = nullptr;
-    cudaError_t e = take_cursor(ctx, n, kBlockRays, &grid, &cursor, &done, stream);
+    cudaError_t e = take_cursor(ctx, n, kBlockRays, kCoopChunk, &grid, &chunk, &cursor, &done, stream);
     if (e != cudaSuccess) return e;
+    if (chunk != kBlockRays) k = any_hit ? k_trace_coop_own<true> : k_trace_coop_own<false>;
     k<<<grid, kCoopBlock, 0, stream>>>(ctx->scene, reinterpret_cast<const float4*>(rays), n,
                                        any_hit ? nullptr : static_cast<uint2*>(out),
-                                       any_hit ? static_cast<uint8_t*>(out) : nullptr, ctx->d_error, cursor);
+                                       any_hit ? static_cast<uint8_t*>(out) : nullptr, ctx->d_error, cursor, chunk);
     if ((e = cudaGetLastError()) != cudaSuccess || !cursor) return e;
     return cudaEventRecord(done, stream);
 }
@@ -463,13 +514,13 @@ static cudaError_t launch_trace_warps(rbr_ctx* ctx, const rbr_ray* rays, uint32_
     // no more warps than there are runs of rays
     uint32_t grid = static_cast<uint32_t>(std::max<uint64_t>(
         1, std::min<uint64_t>(uint64_t(ctx->num_sms) * per_sm, (uint64_t(n) + kPersistBlock - 1) / kPersistBlock)));
-    uint32_t* cursor = nullptr;
+    uint32_t *cursor = nullptr, chunk = 0;
     cudaEvent_t done = nullptr;
-    cudaError_t e = take_cursor(ctx, n, kPersistBlock, &grid, &cursor, &done, stream);
+    cudaError_t e = take_cursor(ctx, n, kPersistBlock, kPersistChunk, &grid, &chunk, &cursor, &done, stream);
     if (e != cudaSuccess) return e;
     e = launch_query(ctx, k, grid, stream, ctx->scene, reinterpret_cast<const float4*>(rays), n, perm,
                      any_hit ? nullptr : static_cast<uint2*>(out), any_hit ? static_cast<uint8_t*>(out) : nullptr,
-                     ctx->d_error, cursor, refill_only ? static_cast<uint32_t>(ctx->trace_refill_min) : kAdaptiveRefill);
+                     ctx->d_error, cursor, chunk, refill_only ? static_cast<uint32_t>(ctx->trace_refill_min) : kAdaptiveRefill);
     return e != cudaSuccess || !cursor ? e : cudaEventRecord(done, stream);
 }
 

@@ -1,0 +1,82 @@
+"""Ray queries captured into a CUDA graph where their hand-out of rays can go wrong: batches around the
+resident blocks' first runs and around the ends of a block's own chunk, against the oracle bit for bit, and
+the captured launch's shape (its blocks claim rays past their first runs, as a plain call's do)."""
+import numpy as np
+import pytest
+import torch
+
+from rbr_b200 import scenes
+
+pytestmark = pytest.mark.gpu
+
+RESIDENT = 148 * 8 * 128  # rays of the first runs of kernels 0 and 1 at 8 blocks per SM
+RESIDENT2 = 148 * 9 * 16  # and of kernel 2 at 9
+
+
+def capture(ctx, rays, any_hit):
+    """The captured graph of one call, and its output buffer (after a plain call that fills it)."""
+    dev = torch.from_numpy(np.frombuffer(rays.tobytes(), np.uint8).copy()).cuda()
+    out = torch.zeros(len(rays) * (1 if any_hit else 8), dtype=torch.uint8, device="cuda")
+    call = ctx.trace_any_dev if any_hit else ctx.trace_closest_dev
+    call(dev.data_ptr(), len(rays), out.data_ptr())
+    torch.cuda.synchronize()
+    plain = out.clone()
+    out.fill_(0xAA)
+    graph = torch.cuda.CUDAGraph(keep_graph=True)
+    with torch.cuda.graph(graph):
+        call(dev.data_ptr(), len(rays), out.data_ptr(), torch.cuda.current_stream().cuda_stream)
+    graph.instantiate()
+    return graph, dev, out, plain
+
+
+def kernel_nodes(graph):
+    driver = pytest.importorskip("cuda.bindings.driver")
+
+    def ok(r):
+        assert r[0] == driver.CUresult.CUDA_SUCCESS
+        return r[1]
+
+    g = driver.CUgraph(graph.raw_cuda_graph())
+    _, _, count = driver.cuGraphGetNodes(g)
+    nodes = ok(driver.cuGraphGetNodes(g, count))
+    return [(n, ok(driver.cuGraphKernelNodeGetParams(n))) for n in nodes
+            if ok(driver.cuGraphNodeGetType(n)) == driver.CUgraphNodeType.CU_GRAPH_NODE_TYPE_KERNEL]
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+@pytest.mark.parametrize("kernel,n", [(k, n) for k in (0, 1) for n in (RESIDENT, RESIDENT + 1, 2 * RESIDENT - 1, 2 * RESIDENT + 1,
+                                                                       3 * RESIDENT + 129, 5 * RESIDENT + 511)]
+                         + [(2, n) for n in (RESIDENT2, RESIDENT2 + 1, 2 * RESIDENT2 + 17, 40 * RESIDENT2 + 255)])
+def test_captured_batches_match_the_oracle(ctx, restatement, kernel, n, any_hit):
+    w = scenes.random_world(30, 150, True, seed=6, flat_triangles=4)
+    ctx.upload(w)
+    rays = scenes.random_test_rays(2 * n + 16, seed=n)[:n]
+    ctx.set_param("trace.kernel", kernel)
+    try:
+        graph, dev, out, plain = capture(ctx, rays, any_hit)
+        graph.replay()
+        torch.cuda.synchronize()
+    finally:
+        ctx.set_param("trace.kernel", 0)
+    assert torch.equal(out, plain)
+    h = restatement.scene(w)
+    got = out.cpu().numpy()
+    if any_hit:
+        assert np.array_equal(got, restatement.trace_any(h, rays))
+    else:
+        want = restatement.trace_closest(h, rays)
+        assert np.array_equal(got.view(np.uint32).reshape(-1, 2)[:, 0], want["prim"].view(np.uint32))
+        assert np.array_equal(got.view(np.uint32).reshape(-1, 2)[:, 1], want["t"].view(np.uint32))
+
+
+@pytest.mark.parametrize("kernel,first_run", [(0, 128), (1, 128), (2, 16)])
+def test_captured_blocks_claim_past_their_first_runs(ctx, kernel, first_run):
+    ctx.upload(scenes.random_world(400, 1500, False, seed=5))
+    n = 1_000_003
+    ctx.set_param("trace.kernel", kernel)
+    try:
+        graph, _, _, _ = capture(ctx, scenes.random_test_rays(2 * n, seed=3)[:n], False)
+        (node, params), = kernel_nodes(graph)
+    finally:
+        ctx.set_param("trace.kernel", 0)
+    assert params.blockDimX == 128 and params.gridDimX * first_run < n
