@@ -128,13 +128,6 @@ rbr_status rbr_ctx_create(int device, rbr_ctx** out) {
         rbr_ctx_destroy(ctx);
         return RBR_ERR_CUDA;
     }
-    for (cudaEvent_t& done : ctx->cursor_done) {
-        if (cudaEventCreateWithFlags(&done, cudaEventDisableTiming) != cudaSuccess) {
-            cudaGetLastError();
-            rbr_ctx_destroy(ctx);
-            return RBR_ERR_CUDA;
-        }
-    }
     *out = ctx;
     return RBR_OK;
 }
@@ -154,8 +147,8 @@ void rbr_ctx_destroy(rbr_ctx* ctx) {
     release(ctx->sort_more[1]);
     if (ctx->d_error) cudaFree(ctx->d_error);
     if (ctx->d_cursors) cudaFree(ctx->d_cursors);
-    for (cudaEvent_t done : ctx->cursor_done)
-        if (done) cudaEventDestroy(done);
+    for (const rbr_ctx::CursorSlot& slot : ctx->cursors)
+        if (slot.done) cudaEventDestroy(slot.done);
     if (ctx->stream) cudaStreamDestroy(ctx->stream);
     if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
     if (ctx->ev_stop) cudaEventDestroy(ctx->ev_stop);

@@ -54,10 +54,14 @@ struct rbr_ctx {
     rbr::DevBuf stage_in, stage_out;
     // device error word (rbr::kErr*)
     int* d_error = nullptr;
-    // work cursors of the persistent trace kernels: one per launch, taken round-robin, and the end of
-    // the launch that used each last
+    // work cursors of the persistent trace kernels: one per launch, taken round-robin, and the stream and
+    // the end of the launch that used each last
+    struct CursorSlot {
+        cudaStream_t stream = nullptr;
+        cudaEvent_t done = nullptr;  // made when the cursor is first taken
+    };
     uint32_t* d_cursors = nullptr;
-    cudaEvent_t cursor_done[rbr::kCursorRing] = {};
+    CursorSlot cursors[rbr::kCursorRing];
     uint32_t cursor_next = 0;
     // tunables (rbr_param_set / rbr_autotune)
     int trace_kernel = 0;          // 0: adaptive persistent warps, 1: warp traversal with lane refill, 2: warp-cooperative

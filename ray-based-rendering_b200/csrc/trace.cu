@@ -441,11 +441,30 @@ __global__ void __launch_bounds__(kCoopBlock, 8)
 
 }  // namespace
 
+// Whether the cursor of `slot` is free for a launch on `stream`: the launch that used it last was on the
+// same stream (the wait for it then costs nothing; should the handle be a destroyed stream's, come back
+// for another one, it orders the two) or is done. The query is allowed while another thread captures in
+// the global mode: the events are never recorded in a capture.
+static cudaError_t cursor_free(rbr_ctx::CursorSlot& slot, cudaStream_t stream, bool* free) {
+    *free = true;
+    if (!slot.done) return cudaEventCreateWithFlags(&slot.done, cudaEventDisableTiming);
+    if (slot.stream == stream) return cudaStreamWaitEvent(stream, slot.done, 0);
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaError_t e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (e != cudaSuccess) return e;
+    const cudaError_t q = cudaEventQuery(slot.done);
+    e = cudaThreadExchangeStreamCaptureMode(&mode);
+    if (q != cudaErrorNotReady) return q != cudaSuccess ? q : e;
+    cudaGetLastError();
+    *free = false;
+    return e;
+}
+
 // How a launch of up to *grid resident blocks with first runs of `block_rays` rays a block hands out n
-// rays: nothing to claim where the first runs are all of them, else a cursor of zero. A cursor of the ring
-// may still be in use by a launch on another stream (64 short launches beside one long one): its event
-// makes `stream` wait for that launch. A launch captured into a graph can run beside any later one, so it
-// gets no cursor: *grid becomes blocks for all rays, each with a chunk of up to `most` first runs of its
+// rays: nothing to claim where the first runs are all of them, else a cursor of zero, the next of the ring.
+// That one may still be in use by a launch on another stream (64 short launches beside one long one), which
+// this call must not wait for, and a launch captured into a graph can run beside any later one: these two
+// get no cursor. *grid becomes blocks for all rays, each with a chunk of up to `most` first runs of its
 // own, so that lanes are refilled within a block and the hardware hands out the blocks. 2^22 uniform rays
 // through 330 K triangles, kernel 0: 1,099 us (951 by a cursor, 1,485 with first runs only, 1,082 with the
 // resident blocks taking runs in turn, which lost a quarter on camera rays: 691 -> 897); kernel 2: 3,560
@@ -459,15 +478,21 @@ static cudaError_t take_cursor(rbr_ctx* ctx, uint32_t n, uint32_t block_rays, ui
     cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
     cudaError_t e = cudaStreamIsCapturing(stream, &capture);
     if (e != cudaSuccess) return e;
-    if (capture != cudaStreamCaptureStatusNone) {
+    const uint32_t at = ctx->cursor_next % kCursorRing;
+    rbr_ctx::CursorSlot& slot = ctx->cursors[at];
+    bool free = capture == cudaStreamCaptureStatusNone;
+    if (free) {
+        ++ctx->cursor_next;
+        if ((e = cursor_free(slot, stream, &free)) != cudaSuccess) return e;
+    }
+    if (!free) {
         *chunk *= std::min(n / (*grid * block_rays), most);
         *grid = static_cast<uint32_t>((uint64_t(n) + *chunk - 1) / *chunk);
         return cudaSuccess;
     }
-    const uint32_t slot = ctx->cursor_next++ % kCursorRing;
-    *done = ctx->cursor_done[slot];
-    if ((e = cudaStreamWaitEvent(stream, *done, 0)) != cudaSuccess) return e;
-    *cursor = ctx->d_cursors + slot;
+    slot.stream = stream;
+    *done = slot.done;
+    *cursor = ctx->d_cursors + at;
     return cudaMemsetAsync(*cursor, 0, sizeof(uint32_t), stream);
 }
 
