@@ -267,10 +267,12 @@ rbr_status rbr_scene_stats_get(const rbr_ctx* ctx, rbr_scene_stats* out);
  *                          set cannot be allocated, the waves run one at a time in the first)
  *   "trace.node_test"      0 or 1; kept for programs that set it: every kernel runs the one node
  *                          test there is
- *   "trace.stream_io"      kernel 0: rays read and hits written with evict-first hints (default 1)
- *   "trace.l2_persist"     kernel 0: 1 reserves the largest persisting-L2 set-aside this process's
- *                          context allows and marks the BVH (nodes and leaf records) persisting for
- *                          each ray-query launch; 0 (default) releases it
+ *   "trace.stream_io"      kernels 0 and 1: rays read and hits written with evict-first hints
+ *                          (default 1; no effect on the small batches that kernel 0 gives to groups
+ *                          of 8 lanes, up to 112 rays per SM)
+ *   "trace.l2_persist"     1 reserves the largest persisting-L2 set-aside this process's context
+ *                          allows and marks the BVH (nodes and leaf records) persisting for each
+ *                          ray-query launch but any-hit ones of sorted rays; 0 (default) releases it
  *   "pt.shade_split"       rbr_render: 1 shades each material class (Lambertian, GGX with a
  *                          Lambertian lobe, GGX reflection only, GGX transmission, delta-only,
  *                          none) in a launch of its own, compiled for that class's lobes; 0 one

@@ -213,7 +213,7 @@ __device__ __forceinline__ uint32_t lane_mask_lt() {
 // waits behind a long one), records tested by their own lane where many lanes have one.
 // With `perm` (sorted rays), position j of the order is ray perm[j]. kRefillOnly: every warp goes
 // the second way.
-constexpr int kPersistBlock = 128;
+constexpr int kPersistBlock = kTraceBlock;
 constexpr uint32_t kPersistChunk = 4;  // first runs in a block's own chunk, at most
 constexpr uint32_t kClaimRays = 32;
 constexpr uint32_t kSmallTree = 64;      // nodes
@@ -365,9 +365,11 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
 
 // ------------------------------------------------------------------------------------------
 // Warp-cooperative traversal: a group of 8 lanes traces one ray (4 rays per warp; group_step in
-// rbr_device.cuh) and takes the next ray of the warp's chunk when its own is done.
+// rbr_device.cuh) and takes the next ray of the warp's chunk when its own is done. Rays and hits go
+// without streaming hints: a small batch's are too few to drive the BVH out of the L2, and with the hints
+// the closest-hit kernel spills.
 // ------------------------------------------------------------------------------------------
-constexpr int kCoopBlock = 128;
+constexpr int kCoopBlock = kTraceBlock;
 constexpr uint32_t kCoopChunk = 16;
 
 template <bool kAny, bool kOwn>
@@ -514,11 +516,10 @@ static cudaError_t launch_trace_coop(rbr_ctx* ctx, const rbr_ray* rays, uint32_t
     cudaError_t e = take_cursor(ctx, n, kBlockRays, kCoopChunk, &grid, &chunk, &cursor, &done, stream);
     if (e != cudaSuccess) return e;
     if (chunk != kBlockRays) k = any_hit ? k_trace_coop_own<true> : k_trace_coop_own<false>;
-    k<<<grid, kCoopBlock, 0, stream>>>(ctx->scene, reinterpret_cast<const float4*>(rays), n,
-                                       any_hit ? nullptr : static_cast<uint2*>(out),
-                                       any_hit ? static_cast<uint8_t*>(out) : nullptr, ctx->d_error, cursor, chunk);
-    if ((e = cudaGetLastError()) != cudaSuccess || !cursor) return e;
-    return cudaEventRecord(done, stream);
+    e = launch_query(ctx, k, grid, stream, ctx->scene, reinterpret_cast<const float4*>(rays), n,
+                     any_hit ? nullptr : static_cast<uint2*>(out), any_hit ? static_cast<uint8_t*>(out) : nullptr,
+                     ctx->d_error, cursor, chunk);
+    return e != cudaSuccess || !cursor ? e : cudaEventRecord(done, stream);
 }
 
 // Kernels 0 (in the given order) and 1: k_trace with the context's parameters.

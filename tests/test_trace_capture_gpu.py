@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 import torch
 
-from rbr_b200 import scenes
+from rbr_b200 import Context, scenes
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +80,25 @@ def test_captured_blocks_claim_past_their_first_runs(ctx, kernel, first_run):
     finally:
         ctx.set_param("trace.kernel", 0)
     assert params.blockDimX == 128 and params.gridDimX * first_run < n
+
+
+@pytest.mark.parametrize("kernel,n", [(0, 1000), (0, 300_001), (1, 300_001), (2, 1000), (2, 300_001)])
+@pytest.mark.parametrize("any_hit", [False, True])
+def test_l2_persist_marks_every_launch(kernel, n, any_hit):
+    """trace.l2_persist reaches small batches (groups of 8 lanes) as it does large ones."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    with Context(0) as ctx:
+        ctx.upload(scenes.random_world(400, 1500, False, seed=5))
+        ctx.set_param("trace.kernel", kernel)
+        rays = scenes.random_test_rays(2 * n, seed=3)[:n]
+        windows = []
+        for on in (0, 1):
+            ctx.set_param("trace.l2_persist", on)
+            graph, _, _, _ = capture(ctx, rays, any_hit)
+            (node, _), = kernel_nodes(graph)
+            err, value = driver.cuGraphKernelNodeGetAttribute(
+                node, driver.CUlaunchAttributeID.CU_LAUNCH_ATTRIBUTE_ACCESS_POLICY_WINDOW)
+            assert err == driver.CUresult.CUDA_SUCCESS
+            windows.append(value.accessPolicyWindow.num_bytes)
+        ctx.set_param("trace.l2_persist", 0)
+    assert windows[0] == 0 and windows[1] > 0
