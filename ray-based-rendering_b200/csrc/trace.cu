@@ -240,11 +240,15 @@ __device__ __forceinline__ bool coherent_pays(const DeviceScene& s, uint32_t n) 
     return n / 32u >= s.num_nodes && (n >= (1u << 20) || s.num_nodes <= kSmallTree);
 }
 
-// Any rays where no lane would be refilled (every ray is in a first run) and the traversals are short:
-// their latency is least one thread per ray (1,001 rays over 260 primitives: 15.1 us against 17.6 by warp
-// traversal).
-__device__ __forceinline__ bool few_rays_small_tree(const DeviceScene& s, bool first_runs_only) {
-    return first_runs_only && s.num_nodes <= kSmallTree;
+// Trees through which any rays are traced one thread per ray, in blocks for all of them without claims:
+// traversals of a few nodes are not worth refilling a lane for, nor 32 of them a claim (those on one cursor
+// are served 0.85 ns apart, 107 us for 2^22 rays). Uniform rays before the persistent warps / by them / so
+// (us): Cornell box (1 node) 2^18 27.7 / 29.7 / 21.6, 2^22 311 / 308 / 234, any hit 219 / 281 / 165;
+// 8 nodes 2^18 23.9 / 25.7 / 17.3, 2^22 250 / 203 / 177; 61 nodes 2^18 58 / 46 / 36, 2^20 191 / 122 / 119,
+// 2^21 363 / 217 / 223: a launch gains by refills from about 2^26 rays times nodes on. Few rays, whose
+// latency counts: 1,001 over 61 nodes 15.1 us, 17.6 by warp traversal.
+__host__ __device__ __forceinline__ bool thread_per_ray(uint32_t num_nodes, uint32_t n) {
+    return num_nodes <= 8u || (num_nodes <= kSmallTree && n <= (1u << 26) / num_nodes);
 }
 
 // The rays a block works on: all n of them, claimed from a cursor that the grid shares, or where there is
@@ -256,7 +260,6 @@ struct BlockRays {
     uint32_t *cursor, *own;
 
     __device__ __forceinline__ uint32_t begin() const { return blockIdx.x * (kOwn && !cursor ? chunk : kBlockRays); }
-    __device__ __forceinline__ bool first_runs_only() const { return !cursor && chunk == kBlockRays; }
     __device__ __forceinline__ void start() const {
         if (!kOwn || cursor || chunk == kBlockRays) return;
         if (threadIdx.x == 0) *own = 0;
@@ -297,7 +300,7 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
     if (run < mine.begin() || run >= n) return;
     uint32_t end = run + min(kClaimRays, n - run);  // warp-uniform
     auto claim = [&]() { return mine.claim(kClaimRays, run, end); };
-    if (!kRefillOnly && (coherent_pays(s, n) || few_rays_small_tree(s, mine.first_runs_only()))) {
+    if (!kRefillOnly && (coherent_pays(s, n) || thread_per_ray(s.num_nodes, n))) {
         uint32_t i = run + lane;
         bool valid = i < end;
         float4 a = make_float4(0.0f, 0.0f, 0.0f, 0.0f), b = a;
@@ -305,7 +308,7 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
             a = ray_word<kStream>(rays + 2 * static_cast<size_t>(i));
             b = ray_word<kStream>(rays + 2 * static_cast<size_t>(i) + 1);
         }
-        if (few_rays_small_tree(s, mine.first_runs_only()) || coherent_rays(s, valid, a, b)) {
+        if (thread_per_ray(s.num_nodes, n) || coherent_rays(s, valid, a, b)) {
             while (true) {
                 if (valid) {
                     float t = 0.0f;
@@ -538,8 +541,9 @@ static cudaError_t launch_trace_warps(rbr_ctx* ctx, const rbr_ray* rays, uint32_
         per_sm = std::max(1, per_sm);
     }
     // no more warps than there are runs of rays
-    uint32_t grid = static_cast<uint32_t>(std::max<uint64_t>(
-        1, std::min<uint64_t>(uint64_t(ctx->num_sms) * per_sm, (uint64_t(n) + kPersistBlock - 1) / kPersistBlock)));
+    const uint64_t all = (uint64_t(n) + kPersistBlock - 1) / kPersistBlock;
+    uint32_t grid = static_cast<uint32_t>(
+        !refill_only && thread_per_ray(ctx->scene.num_nodes, n) ? all : std::min<uint64_t>(uint64_t(ctx->num_sms) * per_sm, all));
     uint32_t *cursor = nullptr, chunk = 0;
     cudaEvent_t done = nullptr;
     cudaError_t e = take_cursor(ctx, n, kPersistBlock, kPersistChunk, &grid, &chunk, &cursor, &done, stream);

@@ -102,3 +102,38 @@ def test_l2_persist_marks_every_launch(kernel, n, any_hit):
             windows.append(value.accessPolicyWindow.num_bytes)
         ctx.set_param("trace.l2_persist", 0)
     assert windows[0] == 0 and windows[1] > 0
+
+
+@pytest.mark.parametrize("ns,nt,n", [(1, 0, 1_000_003), (3, 4, 3_000_001), (10, 30, 1_000_003), (40, 200, 700_001)])
+def test_small_trees_take_one_thread_per_ray(ctx, ns, nt, n):
+    """Over trees of few nodes kernel 0 has a thread for every ray, whatever the batch."""
+    w = scenes.random_world(ns, nt, False, seed=5, flat_triangles=4)
+    ctx.upload(w)
+    nodes = ctx.stats().num_wide_nodes
+    assert nodes <= 8 or (nodes <= 64 and n * nodes <= 1 << 26)
+    graph, _, _, _ = capture(ctx, scenes.random_test_rays(2 * n, seed=3)[:n], False)
+    (_, params), = kernel_nodes(graph)
+    assert params.gridDimX == (n + 127) // 128
+
+
+@pytest.mark.parametrize("any_hit", [False, True])
+@pytest.mark.parametrize("past", [0, 1])
+def test_small_tree_rule_edge_matches_the_oracle(ctx, restatement, past, any_hit):
+    """On both sides of the batch size from which a tree of some 60 nodes goes to warp traversal."""
+    w = scenes.random_world(40, 200, True, seed=5, flat_triangles=4)
+    ctx.upload(w)
+    n = (1 << 26) // ctx.stats().num_wide_nodes + past
+    rays = scenes.random_test_rays(2 * n, seed=7)[:n]
+    chunk = ctx.get_param("trace.host_chunk")
+    ctx.set_param("trace.host_chunk", 0)
+    try:
+        got = ctx.trace_host(rays, any_hit=any_hit)
+    finally:
+        ctx.set_param("trace.host_chunk", chunk)
+    h = restatement.scene(w)
+    if any_hit:
+        assert np.array_equal(got, restatement.trace_any(h, rays))
+    else:
+        want = restatement.trace_closest(h, rays)
+        assert np.array_equal(got["prim"], want["prim"])
+        assert np.array_equal(got["t"].view(np.uint32), want["t"].view(np.uint32))
