@@ -234,10 +234,12 @@ __device__ __forceinline__ bool coherent_rays(const DeviceScene& s, bool valid, 
 
 // Whether one thread per ray pays for coherent rays: where most of a launch is throughput, not the
 // latency of its longest traversals. Camera rays, one thread per ray against warp traversal (us):
-// Cornell box, 2^18 rays 27 / 31, 2^22 131 / 202; 20 K triangles 2^20 121 / 123, 2^21 174 / 198;
-// 405 K 2^20 222 / 191, 2^21 275 / 270, 2^22 390 / 428; 2 M 2^21 437 / 370, 2^22 589 / 540.
+// 20 K triangles 2^20 121 / 123, 2^21 174 / 198; 405 K 2^20 222 / 191, 2^21 275 / 270, 2^22 390 / 428;
+// 2 M 2^21 437 / 370, 2^22 589 / 540. Below 2^20 rays only through small trees, whose longest traversals
+// are short: 109 nodes 2^18 34 / 47, 2^19 59 / 76; 195 nodes 2^18 47 / 63, 2^19 79 / 102; 369 nodes 2^19
+// 117 / 148.
 __device__ __forceinline__ bool coherent_pays(const DeviceScene& s, uint32_t n) {
-    return n / 32u >= s.num_nodes && (n >= (1u << 20) || s.num_nodes <= kSmallTree);
+    return n / 32u >= s.num_nodes && (n >= (1u << 20) || n / 1024u >= s.num_nodes);
 }
 
 // Trees through which any rays are traced one thread per ray, in blocks for all of them without claims:
