@@ -211,11 +211,18 @@ __device__ __forceinline__ uint32_t lane_mask_lt() {
 // traversals of a camera image kept a launch alive behind the others (2^22 rays 1,701 us, 764 at
 // 32). Not kept: claiming the next run ahead of a traversal (679 us instead of 591: a held run
 // waits behind a long one), records tested by their own lane where many lanes have one.
+// An any-hit claim is 64 rays while there are plenty and the last run was quick, since claims on one cursor
+// are served 0.85 ns apart: 2^22 rays that hit the first primitive they meet 106 -> 75 us (20 K triangles,
+// one thread per ray) and 108 -> 90 (2 M, warp traversal), that miss the tree 106 -> 84. It costs other
+// any-hit rays traced one thread per ray 3 % (2^22 through 195 nodes 352 -> 363). Not for closest hits, where a claim of long
+// traversals among quick ones keeps camera images alive: 2^20 rays over 2M triangles 332 -> 379.
 // With `perm` (sorted rays), position j of the order is ray perm[j]. kRefillOnly: every warp goes
 // the second way.
 constexpr int kPersistBlock = kTraceBlock;
 constexpr uint32_t kPersistChunk = 4;  // first runs in a block's own chunk, at most
 constexpr uint32_t kClaimRays = 32;
+constexpr uint32_t kQuickSteps = 3;       // a run of rays that took fewer steps, or by one thread per
+constexpr uint32_t kQuickTicks = 5000;    // ray no more clock ticks, was quick
 constexpr uint32_t kSmallTree = 64;      // nodes
 constexpr uint32_t kAdaptiveRefill = 6;  // idle lanes before a refill (4 to 8 measured within 2 %)
 
@@ -268,6 +275,8 @@ struct BlockRays {
         if (threadIdx.x == 0) *own = 0;
         __syncthreads();
     }
+    // Whether the grid's warps have four more runs each to come.
+    __device__ __forceinline__ bool plenty(uint32_t end) const { return cursor && (n - end) / 4u > gridDim.x * kBlockRays; }
     // The next `count` rays for a warp (run to end); false when there are none. Out of line in kernels with
     // every way of claiming: their code in the traversal loop cost it 1 % (2^22 uniform rays 1,071 -> 1,061 us).
     __device__ __forceinline__ bool claim(uint32_t count, uint32_t& run, uint32_t& end) const {
@@ -307,6 +316,13 @@ struct BlockRays {
     }
 };
 
+// The SM's clock, read no earlier than x is known.
+__device__ __forceinline__ uint32_t clock_after(float x) {
+    uint32_t t;
+    asm volatile("{ .reg .pred p; setp.eq.f32 p, %1, %1; @p mov.u32 %0, %%clock; @!p mov.u32 %0, %%clock; }" : "=r"(t) : "f"(x));
+    return t;
+}
+
 template <bool kAny, bool kStream, bool kRefillOnly>
 __global__ void __launch_bounds__(kPersistBlock, 8)
     k_trace(DeviceScene s, const float4* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ perm,
@@ -321,7 +337,9 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
     uint32_t run = mine.begin() + (threadIdx.x & ~31u);  // warp-uniform
     if (run < mine.begin() || run >= n) return;
     uint32_t end = run + min(kClaimRays, n - run);  // warp-uniform
-    auto claim = [&]() { return mine.claim(kClaimRays, run, end); };
+    auto claim = [&](bool quick = false) {
+        return mine.claim(kAny && quick && mine.plenty(end) ? 2 * kClaimRays : kClaimRays, run, end);
+    };
     if (!kRefillOnly && (coherent_pays(s, n) || thread_per_ray(s.num_nodes, n))) {
         uint32_t i = run + lane;
         bool valid = i < end;
@@ -332,13 +350,17 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
         }
         if (thread_per_ray(s.num_nodes, n) || coherent_rays(s, valid, a, b)) {
             while (true) {
+                uint32_t ticks = 0;
                 if (valid) {
                     float t = 0.0f;
+                    if (kAny && cursor) ticks = clock_after(b.x);
                     const uint32_t r = traverse<kAny>(s, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, t, err);
+                    if (kAny && cursor) ticks = clock_after(__uint_as_float(r)) - ticks;
                     if (kAny) occ[i] = static_cast<uint8_t>(r);
                     else put_hit<kStream>(hits + i, make_uint2(r, r == 0xFFFFFFFFu ? 0u : __float_as_uint(t)));
                 }
-                if (!claim()) return;
+                if (kAny && run + kClaimRays < end) run += kClaimRays;
+                else if (!claim(kAny && !__any_sync(0xFFFFFFFFu, ticks > kQuickTicks))) return;
                 i = run + lane;
                 valid = i < end;
                 if (valid) {
@@ -349,6 +371,7 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
         }
     }
     bool exhausted = false;      // warp-uniform
+    uint32_t steps = 0;          // since the last refill, warp-uniform
     uint32_t idx = 0xFFFFFFFFu;  // this lane's ray
     LaneRay lr;
     uint2 stack[kStackSize];
@@ -367,7 +390,7 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
         // refill once at least refill_min lanes are idle (or all of them): a refill costs the
         // whole warp a few ballots and a ray load, so lanes may idle for a few steps first
         while (need != 0 && !exhausted && (static_cast<uint32_t>(__popc(need)) >= refill_min || need == 0xFFFFFFFFu)) {
-            if (run >= end && !claim()) {
+            if (run >= end && !claim(steps < kQuickSteps && __popc(need) >= 24)) {
                 exhausted = true;
                 break;
             }
@@ -380,10 +403,12 @@ __global__ void __launch_bounds__(kPersistBlock, 8)
                 if (lane_begin<kAny>(s, w, mk(a.x, a.y, a.z), mk(b.x, b.y, b.z), a.w, lr)) answer();
             }
             run = min(end, run + __popc(need));  // each round consumes at least one ray
+            steps = 0;
             need = __ballot_sync(0xFFFFFFFFu, idx == 0xFFFFFFFFu);
         }
         const bool active = idx != 0xFFFFFFFFu;
         if (__ballot_sync(0xFFFFFFFFu, active) == 0) break;  // only when the rays are exhausted
+        ++steps;
         if (warp_step<kAny>(s, w, active, lr, stack, err)) answer();
     }
 }
