@@ -242,9 +242,13 @@ rbr_status rbr_scene_stats_get(const rbr_ctx* ctx, rbr_scene_stats* out);
  *   "trace.kernel"         0 (default): persistent warps that trace coherent rays one thread per
  *                          ray and others by warp traversal (a finished lane takes the next ray,
  *                          leaf records are shared out over the warp), each warp by its own rays;
- *                          one thread per ray where "trace.order" sorts them; 1: warp traversal
- *                          always; 2: warp-cooperative, 8 lanes per ray, one child box per lane
- *   "trace.blocks_per_sm"  resident blocks per SM of kernels 1 and 2 (0: occupancy limit)
+ *                          one thread per ray where "trace.order" sorts them, and through trees
+ *                          of few nodes; small batches through larger trees by groups of 8 lanes;
+ *                          1: warp traversal (batches in the given order that fit the resident
+ *                          warps at once as kernel 0, unless "trace.blocks_per_sm" is set);
+ *                          2: warp-cooperative, 8 lanes per ray, one child box per lane
+ *   "trace.blocks_per_sm"  resident blocks per SM of kernels 1 and 2 (0: occupancy limit); calls
+ *                          captured into a graph have more blocks, each with rays of its own
  *   "trace.refill_min"     kernel 1: idle lanes a warp waits for before it fetches new rays,
  *                          1..32 (default 1: refill after every step with an idle lane)
  *   "trace.min_blocks"     kernel 0 on sorted rays: register budget for 8, 10 or 12 resident

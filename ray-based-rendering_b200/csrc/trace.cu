@@ -214,17 +214,19 @@ __device__ __forceinline__ uint32_t lane_mask_lt() {
 // An any-hit claim is 64 rays while there are plenty and the last run was quick, since claims on one cursor
 // are served 0.85 ns apart: 2^22 rays that hit the first primitive they meet 106 -> 75 us (20 K triangles,
 // one thread per ray) and 108 -> 90 (2 M, warp traversal), that miss the tree 106 -> 84. It costs other
-// any-hit rays traced one thread per ray 3 % (2^22 through 195 nodes 352 -> 363). Not for closest hits, where a claim of long
-// traversals among quick ones keeps camera images alive: 2^20 rays over 2M triangles 332 -> 379.
+// any-hit rays traced one thread per ray 3 % (2^22 through 195 nodes 352 -> 363). Not for closest hits,
+// where a claim of long traversals among quick ones keeps camera images alive: 2^20 rays over 2M triangles
+// 332 -> 379.
 // With `perm` (sorted rays), position j of the order is ray perm[j]. kRefillOnly: every warp goes
 // the second way.
 constexpr int kPersistBlock = kTraceBlock;
+constexpr int kTraceBlocksPerSm = 8;
 constexpr uint32_t kPersistChunk = 4;  // first runs in a block's own chunk, at most
 constexpr uint32_t kClaimRays = 32;
 constexpr uint32_t kQuickSteps = 3;       // a run of rays that took fewer steps, or by one thread per
 constexpr uint32_t kQuickTicks = 5000;    // ray no more clock ticks, was quick
-constexpr uint32_t kSmallTree = 64;      // nodes
-constexpr uint32_t kAdaptiveRefill = 6;  // idle lanes before a refill (4 to 8 measured within 2 %)
+constexpr uint32_t kSmallTree = 64;       // nodes
+constexpr uint32_t kAdaptiveRefill = 6;   // idle lanes before a refill (4 to 8 measured within 2 %)
 
 // Origins within 1/16 of the tree's extent of the warp's first ray's and directions within 11
 // degrees of its: half of a 32-ray run of camera rays spans a degree, rays after a bounce the
@@ -324,7 +326,7 @@ __device__ __forceinline__ uint32_t clock_after(float x) {
 }
 
 template <bool kAny, bool kStream, bool kRefillOnly>
-__global__ void __launch_bounds__(kPersistBlock, 8)
+__global__ void __launch_bounds__(kPersistBlock, kTraceBlocksPerSm)
     k_trace(DeviceScene s, const float4* __restrict__ rays, uint32_t n, const uint32_t* __restrict__ perm,
             uint2* __restrict__ hits, uint8_t* __restrict__ occ, int* err, uint32_t* cursor, uint32_t chunk,
             uint32_t refill_min) {
@@ -578,10 +580,19 @@ static cudaError_t launch_trace_coop(rbr_ctx* ctx, const rbr_ray* rays, uint32_t
     return e != cudaSuccess || !cursor ? e : cudaEventRecord(done, stream);
 }
 
+// Whether the batch is one that never refills a lane in kernel 1 (every ray is in a resident warp's first
+// run). It goes kernel 0's ways, so that a context tuned on large batches traces small ones as well: 33 to
+// 32,768 rays through 61 nodes 19.4 to 21.6 us by kernel 1, 15.3 to 16.6 so; 1,024 through 1.3M triangles 53
+// and 44. Not where the grid or an order is asked for.
+static bool first_runs_only(const rbr_ctx* ctx, uint32_t n) {
+    return ctx->trace_kernel == 1 && ctx->trace_order == 0 && ctx->trace_blocks_per_sm == 0 &&
+           n <= static_cast<uint32_t>(ctx->num_sms) * (kTraceBlocksPerSm * kPersistBlock);
+}
+
 // Kernels 0 (in the given order) and 1: k_trace with the context's parameters.
 static cudaError_t launch_trace_warps(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, void* out,
                                       const uint32_t* perm, cudaStream_t stream) {
-    const bool refill_only = ctx->trace_kernel == 1;
+    const bool refill_only = ctx->trace_kernel == 1 && !first_runs_only(ctx, n);
     const bool st = ctx->trace_stream_io != 0;
     auto k = any_hit ? (refill_only ? (st ? k_trace<true, true, true> : k_trace<true, false, true>)
                                     : (st ? k_trace<true, true, false> : k_trace<true, false, false>))
@@ -694,7 +705,8 @@ cudaError_t launch_trace(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_
     // by groups of 8 lanes: up to 112 rays per SM (16,576) 9 to 25 % faster than by warps of 32 rays
     // on three scenes of 1.3M and 2M triangles (1,024 uniform rays 76 -> 70 us, 8,192 91 -> 78,
     // 8,192 shadow segments 48 -> 40, 16,384 camera rays 185 -> 165).
-    if (ctx->trace_kernel == 0 && ctx->scene.num_nodes > kSmallTree && n <= static_cast<uint32_t>(ctx->num_sms) * 112u)
+    if ((ctx->trace_kernel == 0 || first_runs_only(ctx, n)) && ctx->scene.num_nodes > kSmallTree &&
+        n <= static_cast<uint32_t>(ctx->num_sms) * 112u)
         return launch_trace_coop(ctx, rays, n, any_hit, out, 0, stream);
     const uint32_t* perm = nullptr;  // kernel 1 refills its lanes in sorted order when trace.order is set
     if (ctx->trace_order != 0) {

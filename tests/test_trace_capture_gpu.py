@@ -137,3 +137,26 @@ def test_small_tree_rule_edge_matches_the_oracle(ctx, restatement, past, any_hit
         want = restatement.trace_closest(h, rays)
         assert np.array_equal(got["prim"], want["prim"])
         assert np.array_equal(got["t"].view(np.uint32), want["t"].view(np.uint32))
+
+
+@pytest.mark.parametrize("ns,nt", [(40, 200), (400, 1500)])
+def test_kernel_1_takes_kernel_0s_ways_for_small_batches(ctx, ns, nt):
+    """A batch that never refills a lane runs the same kernel whether kernel 0 or 1 is chosen (by the autotuner)."""
+    driver = pytest.importorskip("cuda.bindings.driver")
+    ctx.upload(scenes.random_world(ns, nt, False, seed=5))
+    names = {}
+    try:
+        for n in (33, 1000, 40_000, RESIDENT, 4 * RESIDENT):
+            rays = scenes.random_test_rays(2 * n + 16, seed=3)[:n]
+            for kernel, per_sm in ((0, 0), (1, 0), (1, 8)):
+                ctx.set_param("trace.kernel", kernel)
+                ctx.set_param("trace.blocks_per_sm", per_sm)
+                graph, _, _, _ = capture(ctx, rays, False)
+                (_, params), = kernel_nodes(graph)
+                names[n, kernel, per_sm] = driver.cuFuncGetName(params.func)[1]
+    finally:
+        ctx.set_param("trace.kernel", 0)
+        ctx.set_param("trace.blocks_per_sm", 0)
+    for n in (33, 1000, 40_000, RESIDENT):
+        assert names[n, 1, 0] == names[n, 0, 0] != names[n, 1, 8]
+    assert names[4 * RESIDENT, 1, 0] != names[4 * RESIDENT, 0, 0]
