@@ -23,18 +23,17 @@ __device__ __forceinline__ float exp2f_approx(float x) {
 }
 
 // Half-width of the band around a byte boundary within which the single-precision estimate below may
-// round the other way. Where encode8's result depends on v, 2^-9 < v^g < 1, so |g log2 v| < 9.1. The
-// approximate logarithm is off by 2^-22 of itself or, for v within [1/2, 2], of 1, so with g <= 4 the
-// exponent is off by at most 9.1 * 2^-22 + 2^-22 (rounding, and 2 ulp of the approximate quotient of
-// the tone map), the approximate power by 2^-22 more: 2.3e-6 of v^g, 5.9e-4 of a byte; 255 p + 0.5 in
-// floats adds half an ulp of 256 twice on either side, 6e-5.
+// round the other way. The approximate logarithm is off by 2^-22 of itself or, for v within [1/2, 2], of
+// 1, so with g <= 4 the exponent g log2 v by 4 x 2^-22 and 5/4 x 2^-22 of itself; the tone map's approximate
+// quotient is off by 2 ulp, at most 2^-22 of v, 5.8 x 2^-22 in the exponent; the power by 2^-22 of itself.
+// A byte x has |g log2 v| = log2(255 / x), and x times the sum (the exponent's by ln 2) is largest at 255:
+// 4.8e-4. 255 p + 0.5 in floats adds half an ulp of 256 twice on either side, 6e-5.
 constexpr float kByteBand = 8e-4f;
 constexpr float kMostInvGamma = 4.0f;
 
-// encode8 of the (tone-mapped) value from approximate functions, or -1 where only the double-precision
-// power decides: within the band of a boundary, for negative values and NaN, and for exponents above
-// kMostInvGamma (band > 1/2: every value).
-__device__ __forceinline__ int encode8_fast(float v, float exposure, float inv_gamma, int tonemap, float band) {
+// encode8 of the (tone-mapped) value from approximate functions, for inv_gamma <= kMostInvGamma, or -1
+// where only the double-precision power decides: within the band of a boundary, for negative values and NaN.
+__device__ __forceinline__ int encode8_fast(float v, float exposure, float inv_gamma, int tonemap) {
     if (tonemap) {
         v *= exposure;
         // below 1e-7 the quotient is v to 2^-23, and the approximate one might flush a subnormal
@@ -42,18 +41,17 @@ __device__ __forceinline__ int encode8_fast(float v, float exposure, float inv_g
     }
     const float p = fminf(exp2f_approx(inv_gamma * __log2f(v)), 1.0f);
     const float x = fmaf(p, 255.0f, 0.5f), f = floorf(x), r = x - f;
-    return v >= 0.0f && r > band && r < 1.0f - band ? static_cast<int>(f) : -1;
+    return v >= 0.0f && r > kByteBand && r < 1.0f - kByteBand ? static_cast<int>(f) : -1;
 }
 
 // Every value of the film on its own: kPer values a thread, as one load and one store where kPer is 4.
-// The double-precision power of every value bound the export (1080p 55 us, 12 times its memory time);
-// with the estimate above one value in 600 still takes it: 16.5 us (22.4 with log2f, exp2f and the
+// The double-precision power of every value bound the export (1080p 56 us, 12 times its memory time);
+// with the estimate above (kFast) one value in 600 still takes it: 17.6 us (22.4 with log2f, exp2f and the
 // exact quotient for every value), bound by the warps in which some value does.
-template <int kPer>
+template <int kPer, bool kFast>
 __global__ void __launch_bounds__(256) k_film_rgb8(const float* __restrict__ film, uint64_t count, float exposure,
                                                    float inv_gamma, int tonemap, uint8_t* __restrict__ out) {
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    const float band = inv_gamma <= kMostInvGamma ? kByteBand : 1.0f;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count / kPer; i += stride) {
         float v[kPer];
         if constexpr (kPer == 4) {
@@ -65,7 +63,7 @@ __global__ void __launch_bounds__(256) k_film_rgb8(const float* __restrict__ fil
         uint32_t word = 0, open = 0;  // bytes, and the values still to encode
 #pragma unroll
         for (int k = 0; k < kPer; ++k) {
-            const int e = encode8_fast(v[k], exposure, inv_gamma, tonemap, band);
+            const int e = kFast ? encode8_fast(v[k], exposure, inv_gamma, tonemap) : -1;
             if (e < 0) open |= 1u << k;
             else word |= static_cast<uint32_t>(e) << (8 * k);
         }
@@ -101,15 +99,22 @@ rbr_status rbr_film_to_rgb8(rbr_ctx* ctx, const float* film, int32_t width, int3
     const float inv_gamma = 1.0f / gamma;
     const auto s = static_cast<cudaStream_t>(stream);
     const uint64_t most = uint64_t(ctx->num_sms) * 32;
-    // four values a thread where the buffers are aligned for it, the last count % 4 one by one
-    const bool wide = (reinterpret_cast<uintptr_t>(film) & 15u) == 0 && (reinterpret_cast<uintptr_t>(out) & 3u) == 0;
+    // Four values a thread where the buffers are aligned for it, the last count % 4 one by one. One value a
+    // thread for small films, which one round of resident threads covers: without a second launch for the
+    // remainder (7x5 16.1 us with it, 11.2 without; no slower at 64x48 to 400x300). Without the estimate for
+    // exponents it does not cover (1080p, gamma 0.2: 58.5 us with it for nothing, 52.4 without).
+    const bool fast = inv_gamma <= kMostInvGamma;
+    const bool wide = fast && count > uint64_t(ctx->num_sms) * 2048 && (reinterpret_cast<uintptr_t>(film) & 15u) == 0 &&
+                      (reinterpret_cast<uintptr_t>(out) & 3u) == 0;
     const uint64_t head = wide ? count & ~uint64_t(3) : 0;
     if (head)
-        k_film_rgb8<4><<<static_cast<uint32_t>(std::min((head / 4 + 255) / 256, most)), 256, 0, s>>>(
+        k_film_rgb8<4, true><<<static_cast<uint32_t>(std::min((head / 4 + 255) / 256, most)), 256, 0, s>>>(
             film, head, exposure, inv_gamma, tonemap, out);
-    if (head < count)
-        k_film_rgb8<1><<<static_cast<uint32_t>(std::min((count - head + 255) / 256, most)), 256, 0, s>>>(
+    if (head < count) {
+        auto k = fast ? k_film_rgb8<1, true> : k_film_rgb8<1, false>;
+        k<<<static_cast<uint32_t>(std::min((count - head + 255) / 256, most)), 256, 0, s>>>(
             film + head, count - head, exposure, inv_gamma, tonemap, out + head);
+    }
     const cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return cuda_fail(ctx, e, "film export");
     return RBR_OK;
