@@ -830,9 +830,13 @@ def main():
     achieved = alg_bytes / avg_launch_s / 1e9
     # DRAM bytes per launch of this very variant from an ncu capture (profiles/traffic.json)
     traffic = None
-    traffic_key = "trace_closest_icosphere8_k{}_b{}_o{}_n{}".format(
-        tuned.get("trace.kernel", 0), ctx.get_param("trace.min_blocks"), tuned.get("trace.order", 0),
-        tuned["trace.node_test"])
+    # (the parameters that matter to it: the refill threshold of kernel 1, the register budget of sorted kernel 0)
+    kernel, order = ctx.get_param("trace.kernel"), ctx.get_param("trace.order")
+    traffic_key = f"trace_closest_icosphere8_k{kernel}_o{order}"
+    if kernel == 1:
+        traffic_key += f"_r{ctx.get_param('trace.refill_min')}"
+    elif kernel == 0 and order:
+        traffic_key += f"_b{ctx.get_param('trace.min_blocks')}"
     tf = REPO / "profiles" / "traffic.json"
     if tf.exists():
         traffic = json.loads(tf.read_text()).get(traffic_key)

@@ -219,12 +219,14 @@ class Context:
         return int(v.value)
 
     def autotune_trace(self, rays_ptr: int, n: int, any_hit: bool = False) -> dict:
-        """Times the traversal variants on these device rays; keeps the fastest. Returns the choice."""
+        """Times the traversal variants on these device rays; keeps the fastest. Returns the choice: every
+        parameter that the autotuner sets, for set_param on another context, and its time."""
         us = C.c_int64()
         self._check(self.lib.rbr_autotune_trace(self.h, C.c_void_p(rays_ptr), n, int(any_hit), C.byref(us)))
         return {"trace.kernel": self.get_param("trace.kernel"), "trace.min_blocks": self.get_param("trace.min_blocks"),
                 "trace.order": self.get_param("trace.order"), "trace.node_test": self.get_param("trace.node_test"),
-                "us_per_launch": us.value}
+                "trace.refill_min": self.get_param("trace.refill_min"),
+                "trace.blocks_per_sm": self.get_param("trace.blocks_per_sm"), "us_per_launch": us.value}
 
     def l2_read_bandwidth(self, nbytes: int = 32 << 20, passes: int = 50) -> float:
         """Read bandwidth (GB/s) of an L2-resident buffer: the traversal roofline's denominator."""
