@@ -260,7 +260,8 @@ def render_scene(which):
 
 
 # Algorithmic bytes of the wavefront path tracer, per event (the fixed record sizes its kernels
-# read and write; traversal bytes come from counted nodes and leaf records, 96 B and 48 B):
+# read and write; traversal bytes come from counted nodes and leaf records, 80 B, the 96 of a node less
+# 16 that repeat its mask of internal slots for every octant, and 48 B):
 #   camera path (k_first: ray 32 + throughput 16 + radiance 16 written, less the queue entry and ray,
 #                36, that depth 0 does not read; k_film: radiance 16)
 #   extension ray (k_first, k_rays: queue 4 + ray 32 + hit 8 + class queue 4)
@@ -270,7 +271,7 @@ def render_scene(which):
 #   shadow ray (k_shade writes and k_rays or k_shadow reads its 48 B record)
 #   pixel (k_film: 12 B of RGB film written)
 PT_BYTES = {"path": 64 - 36 + 16, "extension_ray": 48, "shaded_vertex": 156, "continuation": 52, "shadow_ray": 96,
-            "pixel": 12, "node": 96, "leaf_record": 48}
+            "pixel": 12, "node": 80, "leaf_record": 48}
 
 
 def path_tracer_bytes(st, pixels):
@@ -389,7 +390,8 @@ def measure_render(which, ctx, local_rank, rank, world, steps, warmup, e2e_steps
         "value": paths * world * steps / (total_ms / 1e3) / 1e6, "unit": "Mpaths/s", "steps": steps,
         "warmup": max(3, warmup), "ms_per_step": ms_step, "workload": cfg["desc"], "paths_per_step": paths,
         "e2e": e2e, "cpu_baseline": base, "clocks": clk, "gpu_launches": launches * steps,
-        "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
+        "roofline": {"bound": "issue", "of": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+                     "frac": achieved / peak,
                      "traffic": None, "peak_source": f"{peak_kind} HBM copy bandwidth",
                      "algorithmic_bytes_per_step": alg, "bytes_per_path": alg / paths,
                      "record_bytes": PT_BYTES,
@@ -824,7 +826,7 @@ def main():
     l2_peak = ctx.l2_read_bandwidth(32 << 20, 50)
     # algorithmic traffic of one launch
     nodes, recs = ctx.trace_counts_dev(d_rays.data_ptr(), n)
-    alg_bytes = n * (32 + 8) + nodes * 96 + recs * 48
+    alg_bytes = n * (32 + 8) + nodes * PT_BYTES["node"] + recs * PT_BYTES["leaf_record"]
     avg_launch_s = statistics.mean(launch_ms) / 1e3
     peak, peak_kind = measured_peaks()
     achieved = alg_bytes / avg_launch_s / 1e9
@@ -879,7 +881,7 @@ def main():
             "roofline_l2": {"achieved": achieved, "peak": l2_peak, "unit": "GB/s", "frac": achieved / l2_peak,
                             "peak_source": "read bandwidth of a 32 MiB L2-resident buffer (rbr_l2_read_bandwidth), "
                                            "measured in this run"},
-            "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "roofline": {"bound": "issue", "of": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "traffic": traffic, "traffic_source": traffic_key,
                          "peak_source": f"{peak_kind} HBM copy bandwidth",
                          "algorithmic_bytes_per_launch": alg_bytes,

@@ -325,7 +325,8 @@ rbr_status rbr_trace_host(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any
 /* Diagnostic: replays the traversal of n rays (device pointer) and returns the total number of
  * 8-wide nodes fetched (out[0]) and leaf records tested (out[1]); waits for the result.
  * The traversal order of a ray is deterministic, so these are its algorithmic node and leaf
- * traffic (96 B per node, 48 B per record) for roofline accounting. No reference counterpart. */
+ * traffic for roofline accounting: 96 B fetched per node, 16 of which repeat its mask of internal
+ * slots for every octant, and 48 B per record. No reference counterpart. */
 rbr_status rbr_trace_counts(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int any_hit, uint64_t out[2]);
 
 /* Renders the scene with the wavefront path tracer.

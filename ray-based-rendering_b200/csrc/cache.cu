@@ -913,7 +913,7 @@ __device__ __forceinline__ float adam_update(float p, float& m, float& v, float 
 
 // One Adam step over the MLP weights (dense: FP32 master, BF16 working copy) and the hash-grid entries
 // that received a gradient (entries with a zero gradient keep their parameters and moments); clears the
-// gradients it consumed, and the last block to finish counts the step.
+// gradients it consumed, and counts the step.
 // The grid's scan reads the dense gradient array, four entries a thread and pass; a touched entry's
 // master copy and moments are one 32-byte sector (interleaved state). Bound by the latency of those
 // loads: the states of a thread's touched entries are loaded together, and the next pass's gradients
@@ -978,15 +978,10 @@ __global__ void __launch_bounds__(256) k_rc_adam(AdamDev a, float* master, float
         }
         // (count is a power of two of at least 2^14 entries: no entries past the last group of four)
     }
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        __threadfence();
-        uint32_t* word = reinterpret_cast<uint32_t*>(scalars);
-        if (atomicInc(word + kRcTicket, gridDim.x - 1) == gridDim.x - 1 && c1 != 0.0f) {
-            word[kRcStep] += 1;
-            scalars[kRcLastLoss] = scalars[kRcLoss];
-            scalars[kRcLoss] = 0.0f;
-        }
+    if (first == 0 && c1 != 0.0f) {  // no block of this launch reads these
+        reinterpret_cast<uint32_t*>(scalars)[kRcStep] += 1;
+        scalars[kRcLastLoss] = scalars[kRcLoss];
+        scalars[kRcLoss] = 0.0f;
     }
 }
 

@@ -209,8 +209,8 @@ __device__ __forceinline__ PathKey path_key(const Wave& w, const Paths& P, uint3
 // The counters of depth d.
 __device__ __forceinline__ uint32_t* depth_set(const Paths& P, uint32_t d) { return P.counters + (d & 3u) * kSWords; }
 // Resets them (called by one warp).
-__device__ __forceinline__ void reset_set(const Paths& P, uint32_t d, uint32_t queued = 0) {
-    if (threadIdx.x < kSLines) depth_set(P, d)[threadIdx.x * kLine] = threadIdx.x == 0 ? queued : 0u;
+__device__ __forceinline__ void reset_set(const Paths& P, uint32_t d) {
+    if (threadIdx.x < kSLines) depth_set(P, d)[threadIdx.x * kLine] = 0u;
 }
 
 __device__ __forceinline__ uint32_t lanemask_lt() {

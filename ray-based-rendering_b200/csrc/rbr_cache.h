@@ -90,7 +90,6 @@ enum : int {
     kRcTrain = 6,       // uint32: training vertices appended in this frame
     kRcTrainBase = 7,   // uint32: training count at the start of the current wave
     kRcLastQueries = 8, // uint32: queries of the last frame (summed over waves)
-    kRcTicket = 9,      // uint32: blocks of the optimiser update that have finished
     kRcScalarWords = 16
 };
 

@@ -532,9 +532,9 @@ __device__ __forceinline__ bool test_record(const DeviceScene& s, WarpRays& w, u
 
 // One step of the warp: every lane with `active` tests its node, then the warp tests the records
 // found. Returns true for a lane whose ray is complete.
-template <bool kAny, bool kCount = false>
+template <bool kAny>
 __device__ __forceinline__ bool warp_step(const DeviceScene& s, WarpRays& w, bool active, LaneRay& lr, uint2* stack,
-                                          int* err, uint2* counts = nullptr) {
+                                          int* err) {
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t lt;
     asm("mov.u32 %0, %%lanemask_lt;" : "=r"(lt));
@@ -545,10 +545,6 @@ __device__ __forceinline__ bool warp_step(const DeviceScene& s, WarpRays& w, boo
         uint2 ng = node_group(h);
         recs = leaf_records(h, lr.r.oct);
         prim_base = h.prim_base;
-        if (kCount) {
-            counts->x += 1;
-            counts->y += __popc(recs);
-        }
         if (ng.y < 256u) {
             if (lr.sp == 0) done = true;
             else ng = stack[--lr.sp];  // only non-empty groups are pushed
