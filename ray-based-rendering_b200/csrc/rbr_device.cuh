@@ -151,7 +151,7 @@ __device__ __forceinline__ float hit_record(const DeviceScene& s, uint32_t rec, 
 // The traversal is bound by instruction issue and by the ALU pipe (byte permutes, min / max,
 // compares, mask logic), not by memory, so the test is arranged to issue few of those:
 //   - Slab distances are taken in units of the ray's current limit T, so one saturating FMA per
-//     plane clamps them to [0, 1]: a box is hit if near < far, with no separate comparison
+//     far plane and one saturating product for the near ones clamp them to [0, 1]: a box is hit if near < far, with no separate comparison
 //     against 0 and T (a box behind the origin or past the limit has near = far = 0 or 1).
 //   - near - far is one FADD whose sign bit a funnel shift appends to the hit mask: no compare,
 //     no predicated OR.
@@ -159,7 +159,7 @@ __device__ __forceinline__ float hit_record(const DeviceScene& s, uint32_t rec, 
 //     row its high bit, so the mask comes out in visiting order without a permutation; the node
 //     stores its mask of internal slots permuted for every octant.
 //   - Leaf records are looked up when a leaf slot is visited, not for every slot.
-// 16 instructions per slot (9 on the ALU pipe) where a test with separate clamps that builds the
+// 17 instructions per slot (9 on the ALU pipe) where a test with separate clamps that builds the
 // record mask slot by slot takes 23 (15). Measured against that test: 2^22 uniform rays through
 // 1.3M triangles 1,827 -> 1,430 us, 2M camera rays 607 -> 450 us, 1.5M shadow segments 340 -> 282
 // us, the 1080p GGX render at 64 spp 128.6 -> 106.9 ms, Cornell box 908 -> 884 us (bound by the
@@ -178,7 +178,9 @@ struct RayCtx {
 // kQuantMargin. The widening must not grow with T: 2^-16 of the limit, which for a ray without one is
 // the reach of the whole tree, is more than the leaves of a small mesh in a large scene (330 K triangles
 // of radius 1 over a ground of half size 20,000: 405 nodes and 6,263 records a ray from the mesh where
-// this takes 21 nodes and 125 records; 2^20 rays 84 ms against 2.3).
+// this takes 21 nodes and 125 records; 2^20 rays 84 ms against 2.3). One product per slot with the largest
+// near distance: scaled factors and offsets of the planes take six registers more, and the path tracer's
+// kernels spill (64x48 preview 153.8 us, 148.4 so; 2^22 uniform rays 1,039 and 1,044).
 constexpr float kNearScale = 1.0f - 1.0f / 65536.0f;
 
 __device__ __forceinline__ float rcp_approx(float x) {
@@ -234,6 +236,12 @@ __device__ __forceinline__ float fma_sat(float a, float b, float c) {
     return d;
 }
 
+__device__ __forceinline__ float mul_sat(float a, float b) {
+    float d;
+    asm("mul.rn.sat.f32 %0, %1, %2;" : "=f"(d) : "f"(a), "f"(b));
+    return d;
+}
+
 // Three-input minimum / maximum (sm_100).
 __device__ __forceinline__ float fmax3(float a, float b, float c) {
     float d;
@@ -272,8 +280,7 @@ struct NodeHits {
 // b comes from one FMA of p with the ray's o / (d T): its rounding error, 2^-24 o / d, stays below
 // the 2^-20 of the scene's largest coordinate every box is padded with, plus the widening in t.
 struct NodeView {
-    float nax, nay, naz, nx, ny, nz;                    // near planes: factors, offsets
-    float ax, ay, az, fx, fy, fz;                       // far planes
+    float ax, ay, az, bx, by, bz;                       // factors, offsets
     uint32_t px[2], Px[2], py[2], Py[2], pz[2], Pz[2];  // near (p) and far (P) plane bytes, 8 slots
 };
 
@@ -285,15 +292,9 @@ __device__ __forceinline__ NodeView node_view(const uint4* __restrict__ nodes, u
     v.ax = __uint_as_float(C.w[6] << 16) * r.ix;
     v.ay = __uint_as_float(C.w[6] & 0xFFFF0000u) * r.iy;
     v.az = __uint_as_float(C.w[7]) * r.iz;
-    v.fx = fmaf(__uint_as_float(A.w[0]), r.ix, -r.qx);
-    v.fy = fmaf(__uint_as_float(A.w[1]), r.iy, -r.qy);
-    v.fz = fmaf(__uint_as_float(A.w[2]), r.iz, -r.qz);
-    v.nax = v.ax * kNearScale;
-    v.nay = v.ay * kNearScale;
-    v.naz = v.az * kNearScale;
-    v.nx = v.fx * kNearScale;
-    v.ny = v.fy * kNearScale;
-    v.nz = v.fz * kNearScale;
+    v.bx = fmaf(__uint_as_float(A.w[0]), r.ix, -r.qx);
+    v.by = fmaf(__uint_as_float(A.w[1]), r.iy, -r.qy);
+    v.bz = fmaf(__uint_as_float(A.w[2]), r.iz, -r.qz);
     const bool sx = r.oct & 1u, sy = r.oct & 2u, sz = r.oct & 4u;
 #pragma unroll
     for (int w = 0; w < 2; ++w) {
@@ -315,11 +316,11 @@ __device__ __forceinline__ NodeView node_view(const uint4* __restrict__ nodes, u
 
 // near - far of the slot whose plane bytes lie in word w at selector sel: negative if hit.
 __device__ __forceinline__ float slot_gap(const NodeView& v, int w, uint32_t sel) {
-    const float n = fmax3(fma_sat(qplane(v.px[w], sel), v.nax, v.nx), fma_sat(qplane(v.py[w], sel), v.nay, v.ny),
-                          fma_sat(qplane(v.pz[w], sel), v.naz, v.nz));
-    const float f = fmin3(fma_sat(qplane(v.Px[w], sel), v.ax, v.fx), fma_sat(qplane(v.Py[w], sel), v.ay, v.fy),
-                          fma_sat(qplane(v.Pz[w], sel), v.az, v.fz));
-    return n - f;
+    const float n = fmax3(fmaf(qplane(v.px[w], sel), v.ax, v.bx), fmaf(qplane(v.py[w], sel), v.ay, v.by),
+                          fmaf(qplane(v.pz[w], sel), v.az, v.bz));
+    const float f = fmin3(fma_sat(qplane(v.Px[w], sel), v.ax, v.bx), fma_sat(qplane(v.Py[w], sel), v.ay, v.by),
+                          fma_sat(qplane(v.Pz[w], sel), v.az, v.bz));
+    return mul_sat(n, kNearScale) - f;
 }
 
 // Tests the 8 children of node `idx`.
