@@ -336,7 +336,8 @@ rbr_status rbr_trace_counts(rbr_ctx* ctx, const rbr_ray* rays, uint32_t n, int a
  * of squared sample values (width*height*3 floats). Asynchronous on `stream`: with
  * "pt.streams" 2 every other wave runs on a second stream of the context that forks from
  * `stream` at the start and joins it at the end, so work queued on `stream` afterwards sees
- * the whole film.
+ * the whole film. Calls with the same arguments render the same bits for scenes of at most one
+ * light; a path's samples of several lights are added in the order in which they finish.
  * Replaces: Integrator::render with PathTracingIntegrator::Li (src/renderers/integrator.cpp:7-50,
  * src/renderers/path_tracing_integrator.cpp:5-138). */
 rbr_status rbr_render(rbr_ctx* ctx, const rbr_camera* camera, const rbr_render_params* params,

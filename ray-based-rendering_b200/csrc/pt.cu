@@ -245,8 +245,9 @@ __device__ __forceinline__ bool degenerate(float4 o, float4 d) {
 // ------------------------------------------------------------------------------------------
 // Whether a stage that traverses rays hands out a long queue by claims: only through a tree of more than
 // kClaimNodes nodes. In a few nodes every ray costs about the same and so little that warps wait for
-// their claims (us, grid stride / claims: Cornell box at 64 spp 2,677 / 3,775, foggy 4,908 / 7,859;
-// material scene of 800 triangles and 256 spheres 5,956 / 5,540, of 2M triangles 94,753 / 89,637).
+// their claims. Renders of 512 x 512 at 64 spp, by nodes, grid stride / claims (ms): surface 1 node 3.90 /
+// 4.10, 5 4.78 / 4.79, 17 5.27 / 5.14, 51 7.67 / 7.17, 79 10.24 / 9.40, 391 11.03 / 10.11; in fog 1 node 22.1 /
+// 26.7, 51 27.3 / 30.4, 79 30.3 / 32.1, 127 32.7 / 33.7, 391 30.7 / 33.0. 2M triangles 94.8 / 89.6.
 constexpr uint32_t kClaimNodes = 64;
 __device__ __forceinline__ bool claims_pay(const DeviceScene& s, const Paths& P) {
     return P.fetch != 0 && s.num_nodes > kClaimNodes;
