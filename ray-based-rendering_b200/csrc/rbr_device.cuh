@@ -180,7 +180,8 @@ struct RayCtx {
 // of radius 1 over a ground of half size 20,000: 405 nodes and 6,263 records a ray from the mesh where
 // this takes 21 nodes and 125 records; 2^20 rays 84 ms against 2.3). One product per slot with the largest
 // near distance: scaled factors and offsets of the planes take six registers more, and the path tracer's
-// kernels spill (64x48 preview 153.8 us, 148.4 so; 2^22 uniform rays 1,039 and 1,044).
+// kernels spill (256x256 Cornell box, 16 spp, 722 us, 719 so; 64x48 preview 154 both; 2^22 uniform rays
+// 1,039 and 1,044).
 constexpr float kNearScale = 1.0f - 1.0f / 65536.0f;
 
 __device__ __forceinline__ float rcp_approx(float x) {
